@@ -30,6 +30,7 @@ UNITS = [
     ("lib/api.cu", ["--fmad=false"]),
     ("lib/k_particles.cu", ["--fmad=false"]),
     ("lib/k_field.cu", ["--fmad=false"]),
+    ("lib/k_deposit.cu", ["--fmad=false"]),
     ("lib/k_load.cu", ["--fmad=false"]),
     ("lib/k_1d.cu", ["--fmad=false"]),
     ("lib/k_wake.cu", ["--fmad=false"]),

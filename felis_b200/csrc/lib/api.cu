@@ -73,7 +73,11 @@ struct felis_handle {
   DevDeposit dep{};
   int64_t dep_cap = 0;
   bool has_even = false;
-  int dep_pcap = 0;
+  DepositPlan dep_plan{};
+  // radial elimination of the lattice constant radial_A (NaN: none yet); the
+  // launches that write and read it are in stream order
+  double2* d_radial = nullptr;
+  double radial_A = NAN;
   // field
   double2* U = nullptr;
   double2* Sc = nullptr;
@@ -467,13 +471,19 @@ felis_status run_deposit(felis_handle* h, const felis_lattice& L) {
   }
   const double ks = h->p.ks, ue = L.ue, K0 = L.K0, gamR = h->p.gam_r, dr = h->p.dr;
   d.A = ks * ks * (1.0 + 0.5 * (1.0 + ue * ue) * K0 * K0) / (gamR * gamR) * dr * dr;
-  d.cap = h->dep_pcap;
+  d.chunk2 = h->dep_plan.chunk2;
+  d.chunkr = h->dep_plan.chunkr;
+  d.radial = h->d_radial;
   d.neven = 0;
   for (int k = 0; k < h->p.num_harmony; ++k) d.neven += (h->p.harmony[k] % 2 == 0);
   d.err = h->d_err;
   {
     KernelScope ks(h, FELIS_KERNEL_DEPOSIT);
-    launch_deposit(d, h->st);
+    if (!(h->radial_A == d.A)) {
+      launch_radial_elimination(d.A, h->p.scl_mode, h->p.scf_mode, h->p.nr, h->d_log, h->d_radial, h->st);
+      h->radial_A = d.A;
+    }
+    launch_deposit(d, h->dep_plan.smem, h->st);
   }
   CK(cudaGetLastError());
   return FELIS_OK;
@@ -544,12 +554,6 @@ felis_status relayout(felis_handle* h, const std::vector<int64_t>& new_counts_pe
   h->soff = soff;
   // tiles
   h->tiles.clear();
-  int64_t maxslice = 0;
-  for (int s = 0; s < S; ++s) {
-    int64_t c = 0;
-    for (int sp = 0; sp < ns; ++sp) c += soff[(size_t)sp * (S + 1) + s + 1] - soff[(size_t)sp * (S + 1) + s];
-    maxslice = std::max(maxslice, c);
-  }
   for (int sp = 0; sp < ns; ++sp)
     for (int s = 0; s < S; ++s) {
       const int64_t b = soff[(size_t)sp * (S + 1) + s], e = soff[(size_t)sp * (S + 1) + s + 1];
@@ -586,26 +590,13 @@ felis_status relayout(felis_handle* h, const std::vector<int64_t>& new_counts_pe
     CK(cudaMalloc(&h->dep.ez, n * LF * sizeof(double2)));
     h->dep_cap = n;
   }
-  // deposit chunk: the largest power of two (<= 4096 particles) whose sort
-  // buffers and records fit in ~100 KB of shared memory (two CTAs per SM)
   int dev_smem = 0;
   cudaDeviceGetAttribute(&dev_smem, cudaDevAttrMaxSharedMemoryPerBlockOptin, h->device);
-  const size_t budget = std::min<size_t>(100 * 1024, (size_t)dev_smem);
-  const int H = h->p.num_harmony, Lm = h->p.scl_mode, Fm = h->p.scf_mode, nr = h->p.nr;
   int neven = 0;
-  for (int k = 0; k < H; ++k) neven += (h->p.harmony[k] % 2 == 0);
-  int cap = 4096;
-  while (cap > 64 && deposit_smem_bytes(cap, H, neven, Lm, Fm, nr) > budget) cap >>= 1;
-  const size_t smem = deposit_smem_bytes(cap, H, neven, Lm, Fm, nr);
-  if ((int)smem > dev_smem) return fail(h, FELIS_UNSUPPORTED, "deposit buffers do not fit in shared memory");
-  int qb = 0;
-  while ((1 << qb) < cap) ++qb;
-  int kb = 0;
-  while ((1 << kb) < h->p.nx * h->p.ny + 1) ++kb;
-  if (kb + qb > 32) return fail(h, FELIS_UNSUPPORTED, "grid too large for 32-bit deposit keys");
-  deposit_set_smem(smem);
-  h->dep_pcap = cap;
-  (void)maxslice;
+  for (int k = 0; k < h->p.num_harmony; ++k) neven += (h->p.harmony[k] % 2 == 0);
+  if (!deposit_plan(h->p.num_harmony, neven, h->p.scl_mode, h->p.scf_mode, h->p.nr, (size_t)dev_smem, &h->dep_plan))
+    return fail(h, FELIS_UNSUPPORTED, "deposit buffers do not fit in shared memory");
+  deposit_set_smem(h->dep_plan.smem);
   invalidate_particles(h);
   return FELIS_OK;
 }
@@ -724,6 +715,7 @@ felis_status felis_create(const felis_params* p, felis_handle** out) {
   std::vector<double> logtab(p->nr, 0.0);
   for (int j = 1; j < p->nr; ++j) logtab[j] = log((j + 0.5) / (j - 0.5));
   if (ce == cudaSuccess) ce = cudaMalloc(&h->d_log, logtab.size() * sizeof(double));
+  if (ce == cudaSuccess) ce = cudaMalloc(&h->d_radial, (size_t)p->scl_mode * p->scf_mode * p->nr * sizeof(double2));
   if (ce == cudaSuccess) ce = cudaMemcpy(h->d_log, logtab.data(), logtab.size() * sizeof(double), cudaMemcpyHostToDevice);
   if (ce == cudaSuccess) ce = cudaMalloc(&h->d_planes, (size_t)H * 2 * S * sizeof(double));
   if (ce == cudaSuccess) ce = cudaMalloc(&h->d_planes2, (size_t)H * 2 * S * sizeof(double));
@@ -818,7 +810,7 @@ void felis_destroy(felis_handle* h) {
   if (!h) return;
   if (h->st) cudaStreamSynchronize(h->st);
   void* ptrs[] = {h->x, h->y, h->px, h->py, h->th, h->ga, h->d_soff, h->d_weight, h->d_tiles, h->U, h->Sc, h->box,
-                  h->Ez, h->d_bessel, h->d_wake, h->d_log, h->d_adi, h->d_part, h->d_planes, h->d_planes2,
+                  h->Ez, h->d_bessel, h->d_wake, h->d_log, h->d_radial, h->d_adi, h->d_part, h->d_planes, h->d_planes2,
                   h->d_hist_e, h->d_hist_t, h->d_hist_b, h->d_tmp, h->d_l1, h->d_err,
                   h->dep.key, h->dep.rkey, h->dep.wx1, h->dep.wy1, h->dep.wr1, h->dep.coef, h->dep.fx, h->dep.fy, h->dep.ez,
                   h->adi_scratch};
@@ -1292,10 +1284,14 @@ felis_status felis_run(felis_handle* h, int32_t it0, int32_t it1) {
   h->capturing = false;
   cudaError_t ce = cudaStreamEndCapture(h->st, &graph);
   if (s != FELIS_OK) {
+    h->radial_A = NAN;  // the captured launches did not run
     if (graph) cudaGraphDestroy(graph);
     return s;
   }
-  if (ce != cudaSuccess) return fail(h, FELIS_CUDA_ERROR, std::string("graph capture: ") + cudaGetErrorString(ce));
+  if (ce != cudaSuccess) {
+    h->radial_A = NAN;
+    return fail(h, FELIS_CUDA_ERROR, std::string("graph capture: ") + cudaGetErrorString(ce));
+  }
   ce = cudaGraphInstantiate(&exec, graph, 0);
   cudaEvent_t e0 = nullptr, e1 = nullptr;
   if (ce == cudaSuccess) ce = cudaEventCreate(&e0);
@@ -1313,7 +1309,10 @@ felis_status felis_run(felis_handle* h, int32_t it0, int32_t it1) {
   if (e1) cudaEventDestroy(e1);
   if (exec) cudaGraphExecDestroy(exec);
   cudaGraphDestroy(graph);
-  if (ce != cudaSuccess) return fail(h, FELIS_CUDA_ERROR, std::string("graph run: ") + cudaGetErrorString(ce));
+  if (ce != cudaSuccess) {
+    h->radial_A = NAN;
+    return fail(h, FELIS_CUDA_ERROR, std::string("graph run: ") + cudaGetErrorString(ce));
+  }
   return check_err(h);
 }
 

@@ -105,7 +105,7 @@ struct DevParticles {
 
 // Per-particle deposit records (written before the ordered deposit).
 struct DevDeposit {
-  int* key;        // idxJ*nx + idxI, or -1
+  int* key;        // idxJ << 16 | idxI, or -1
   int* rkey;       // idxR (0 <= idxR < nr), or -1
   double* wx1;     // wx[1]
   double* wy1;     // wy[1]

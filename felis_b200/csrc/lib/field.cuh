@@ -47,13 +47,23 @@ struct DepositLaunch {
   double2 fconst[FELIS_MAX_HARMONY][2];  // odd-harmonic fx, fy (per call constants)
   cd etaX, etaY;
   double A;             // Ez Thomas coefficient (solveField.cpp:320)
-  int cap;              // particles per chunk (<= 4096, the radix sort's u16 counters)
   int neven;            // number of even harmonics
+  int chunk2, chunkr;   // particles per chunk of the 2-D and the radial sums (DepositPlan)
+  const double2* radial;  // [L*F][nr] radial elimination for A (launch_radial_elimination)
   int* err;
 };
 
-void launch_deposit(const DepositLaunch& a, cudaStream_t st);
-size_t deposit_smem_bytes(int chunk, int H, int neven, int L, int F, int nr);
+// Chunk sizes and shared memory of the deposit; false when the radial grid is
+// too large for it.
+struct DepositPlan {
+  int chunk2 = 0, chunkr = 0;
+  size_t smem = 0;
+};
+bool deposit_plan(int H, int neven, int L, int F, int nr, size_t dev_smem, DepositPlan* p);
+void launch_deposit(const DepositLaunch& a, size_t smem, cudaStream_t st);
+// Multiplier and pivot of every point and mode of the radial Ez solve with
+// the coefficient A (DepositLaunch::A): L * F <= 16 modes.
+void launch_radial_elimination(double A, int L, int F, int nr, const double* logtab, double2* out, cudaStream_t st);
 void deposit_set_smem(size_t bytes);
 void adi_set_smem(size_t bytes);
 void launch_adi(const AdiLaunch& a, cudaStream_t st);

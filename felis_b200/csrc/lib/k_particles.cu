@@ -282,7 +282,7 @@ __device__ __forceinline__ void prep_one(const ParticleLaunch& a, int64_t n, dou
   D.wx1[n] = (x - G.minX) / G.dx - idxI;
   D.wy1[n] = (y - G.minY) / G.dy - idxJ;
   const bool in = idxI >= 0 && idxI < nx && idxJ >= 0 && idxJ < ny;
-  D.key[n] = in ? idxJ * nx + idxI : -1;
+  D.key[n] = in ? idxJ << 16 | idxI : -1;
   if (in && (idxI == nx - 1 || idxJ == ny - 1)) atomicAdd(a.err + ERR_EDGE_DEPOSIT, 1);
   if (in) {
     for (int h = 0; h < G.H; ++h) {
