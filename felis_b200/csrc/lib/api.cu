@@ -777,11 +777,12 @@ felis_status felis_create(const felis_params* p, felis_handle** out) {
     if (st == FELIS_OK && (int)smem <= dev_smem - 1024) {
       adi_set_smem(smem);
     } else if (st == FELIS_OK) {
-      // plane larger than shared memory: global-memory sweeps, one scratch
-      // plane per CTA of a persistent grid
+      // plane larger than shared memory: swept in tiles, one scratch plane per
+      // CTA of a persistent grid
       h->adi_big_grid = std::min(S * H * 2, h->sms * 2);
       if (cudaMalloc(&h->adi_scratch, (size_t)h->adi_big_grid * nx * ny * sizeof(double2)) != cudaSuccess)
         bail(FELIS_CUDA_ERROR, "ADI scratch allocation failed");
+      adi_big_set_smem(adi_big_smem_bytes(nx, ny));
     }
     if (st == FELIS_OK && std::max(nx, ny) > 256) bail(FELIS_UNSUPPORTED, "grid wider than 256 points");
   }
