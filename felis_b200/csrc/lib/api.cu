@@ -251,7 +251,9 @@ bool trans_coef(const felis_handle* h, const felis_lattice& L, TransCoef* t) {
   t->xCoef = 0.0;
   t->yCoef = 0.0;
   t->K0_alpha = L.K0_alpha;
-  t->valid = 1;
+  t->fast = 1;
+  for (double v : {t->dz, t->ku, t->K0, t->ue, t->aa, t->bb, t->cc})
+    if (!(v == 0.0 || (fabs(v) > 0x1p-60 && fabs(v) < 0x1p60))) t->fast = 0;
   if (L.und_type == FELIS_BIPOLAR) {
     if (L.K0_alpha == 1) { t->xCoef = 1; t->yCoef = 0; }
     else if (L.K0_alpha == -1) { t->xCoef = 0; t->yCoef = 1; }

@@ -26,7 +26,7 @@ enum ParticleOps : unsigned {
 struct TransCoef {
   double dz, ku, K0, ue, aa, bb, cc, xCoef, yCoef;
   int K0_alpha;
-  int valid;
+  int fast;  // every coefficient is zero or of ordinary size (k_particles.cu, within)
 };
 
 // particlePush.cpp:213-244 / 124-139 scalars of one push or drift call.
