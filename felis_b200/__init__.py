@@ -385,10 +385,9 @@ class Handle:
         self._ck(_lib.felis_upload_field(self._h, hidx, pol, _p(buf)))
 
     def _dl(self, fn, hidx, pol) -> np.ndarray:
-        n = (self.S + 2) * self.nx * self.ny
-        buf = np.zeros(2 * n)
+        buf = np.empty(2 * (self.S + 2) * self.nx * self.ny)
         self._ck(fn(self._h, hidx, pol, _p(buf)))
-        return (buf[0::2] + 1j * buf[1::2]).reshape(self.S + 2, self.ny, self.nx)
+        return buf.view(np.complex128).reshape(self.S + 2, self.ny, self.nx)
 
     def download_field(self, hidx: int, pol: int) -> np.ndarray:
         return self._dl(_lib.felis_download_field, hidx, pol)
@@ -600,9 +599,9 @@ class Batch:
 
     def download_field(self, inst: int, hidx: int, pol: int) -> np.ndarray:
         S, nx, ny = self.S[inst], self.nx[inst], self.ny[inst]
-        buf = np.zeros(2 * (S + 2) * nx * ny)
+        buf = np.empty(2 * (S + 2) * nx * ny)
         self._ck(_lib.felis_batch_download_field(self._b, inst, hidx, pol, _p(buf)))
-        return (buf[0::2] + 1j * buf[1::2]).reshape(S + 2, ny, nx)
+        return buf.view(np.complex128).reshape(S + 2, ny, nx)
 
     def run(self, it0: int, it1: int):
         self._ck(_lib.felis_batch_run(self._b, it0, it1))
@@ -724,7 +723,7 @@ class MLP:
 
     def forward(self, x) -> np.ndarray:
         x = _f32(x).reshape(-1, self.n_in)
-        y = np.zeros((x.shape[0], self.n_out), dtype=np.float32)
+        y = np.empty((x.shape[0], self.n_out), dtype=np.float32)
         self._ck(_lib.felis_mlp_forward(self._m, _pf(x), x.shape[0], _pf(y)))
         return y
 

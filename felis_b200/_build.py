@@ -36,6 +36,7 @@ UNITS = [
     ("lib/k_wake.cu", ["--fmad=false"]),
     ("lib/k_sort.cu", []),
     ("lib/batch.cu", []),
+    ("lib/transfer.cu", []),
     ("lib/k_batch.cu", ["--use_fast_math"]),
     ("lib/mlp.cu", []),
     ("lib/k_mlp.cu", []),

@@ -25,6 +25,7 @@
 #include "field.cuh"
 #include "oned.cuh"
 #include "particles.cuh"
+#include "transfer.cuh"
 
 using namespace felis;
 
@@ -126,6 +127,7 @@ struct felis_handle {
   // slice sharding across processes: the shift leaves the plane that becomes
   // the first slice holding the old last slice, for the caller to exchange
   bool exchange = false;
+  HostStage stage;  // field downloads
 };
 
 namespace {
@@ -902,9 +904,14 @@ felis_status felis_upload_field(felis_handle* h, int32_t hidx, int32_t pol, cons
   if (!h || hidx < 0 || hidx >= h->p.num_harmony || pol < 0 || pol > 1 || !data) return fail(h, FELIS_BAD_ARG, "bad argument");
   const int S = h->p.slice_n;
   const size_t N = (size_t)h->p.nx * h->p.ny;
-  for (int s = 0; s < S; ++s)
-    CK(cudaMemcpyAsync(h->U + field_plane(S, hidx, pol, s, h->ring_base) * N, data + 2 * (size_t)(s + 1) * N,
-                       N * sizeof(double2), cudaMemcpyHostToDevice, h->st));
+  // the ring holds the slices in two runs of planes
+  const int run = S - h->ring_base;  // slices 0 .. run - 1 sit at ring_base ..
+  double2* P = h->U + (size_t)(hidx * 2 + pol) * S * N;
+  CK(cudaMemcpyAsync(P + (size_t)h->ring_base * N, data + 2 * N, (size_t)run * N * sizeof(double2),
+                     cudaMemcpyHostToDevice, h->st));
+  if (run < S)
+    CK(cudaMemcpyAsync(P, data + 2 * (size_t)(run + 1) * N, (size_t)(S - run) * N * sizeof(double2),
+                       cudaMemcpyHostToDevice, h->st));
   CK(cudaStreamSynchronize(h->st));
   h->diag_valid = false;
   return FELIS_OK;
@@ -916,9 +923,18 @@ felis_status felis_download_field(felis_handle* h, int32_t hidx, int32_t pol, do
   const size_t N = (size_t)h->p.nx * h->p.ny;
   memset(data, 0, 2 * N * sizeof(double));
   memset(data + 2 * (size_t)(S + 1) * N, 0, 2 * N * sizeof(double));
-  for (int s = 0; s < S; ++s)
-    CK(cudaMemcpyAsync(data + 2 * (size_t)(s + 1) * N, h->U + field_plane(S, hidx, pol, s, h->ring_base) * N,
-                       N * sizeof(double2), cudaMemcpyDeviceToHost, h->st));
+  const int run = S - h->ring_base;
+  const double2* P = h->U + (size_t)(hidx * 2 + pol) * S * N;
+  const CopyPart parts[2] = {{P + (size_t)h->ring_base * N, data + 2 * N, (size_t)run * N * sizeof(double2)},
+                                 {P, data + 2 * (size_t)(run + 1) * N, (size_t)(S - run) * N * sizeof(double2)}};
+  cudaPointerAttributes at{};
+  if (cudaPointerGetAttributes(&at, data) == cudaSuccess && at.type == cudaMemoryTypeHost) {
+    for (const CopyPart& p : parts)
+      if (p.bytes) CK(cudaMemcpyAsync(p.dst, p.src, p.bytes, cudaMemcpyDeviceToHost, h->st));
+  } else {
+    cudaGetLastError();
+    CK(h->stage.download(parts, 2, false, h->device, h->st));
+  }
   CK(cudaStreamSynchronize(h->st));
   return FELIS_OK;
 }

@@ -25,6 +25,7 @@
 #include <vector>
 
 #include "batch.cuh"
+#include "transfer.cuh"
 
 using namespace felis;
 
@@ -346,6 +347,7 @@ struct felis_batch {
   // copied as they are and rounded or widened on the device)
   double* stage = nullptr;
   size_t stage_bytes = 0;
+  HostStage host_stage;  // field downloads
 };
 
 namespace {
@@ -963,17 +965,17 @@ felis_status felis_batch_download_field(felis_batch* b, int32_t inst, int32_t hi
   if (!b || inst < 0 || inst >= (int)b->in.size() || !data) return bfail(b, FELIS_BAD_ARG, "bad argument");
   Inst& I = b->in[inst];
   if (hidx < 0 || hidx >= I.p.num_harmony || pol < 0 || pol > 1) return bfail(b, FELIS_BAD_ARG, "bad harmonic/pol");
-  BCK(cudaStreamSynchronize(b->st));
   const int S = I.p.slice_n;
   const size_t N = (size_t)I.p.nx * I.p.ny;
-  std::vector<float2> plane(N);
-  memset(data, 0, 2 * (size_t)(S + 2) * N * sizeof(double));
-  for (int s = 0; s < S; ++s) {
-    const int phys = (s + I.ring_base) % S;
-    BCK(cudaMemcpy(plane.data(), I.U + ((size_t)(hidx * 2 + pol) * S + phys) * N, N * sizeof(float2), cudaMemcpyDeviceToHost));
-    double* dst = data + 2 * (size_t)(s + 1) * N;
-    for (size_t k = 0; k < N; ++k) { dst[2 * k] = plane[k].x; dst[2 * k + 1] = plane[k].y; }
-  }
+  memset(data, 0, 2 * N * sizeof(double));
+  memset(data + 2 * (size_t)(S + 1) * N, 0, 2 * N * sizeof(double));
+  // the ring holds the slices in two runs of planes; they cross the link in
+  // FP32 and are widened on the way into the caller's array
+  const int run = S - I.ring_base;
+  const float2* P = I.U + (size_t)(hidx * 2 + pol) * S * N;
+  const CopyPart parts[2] = {{P + (size_t)I.ring_base * N, data + 2 * N, (size_t)run * N * sizeof(float2)},
+                                 {P, data + 2 * (size_t)(run + 1) * N, (size_t)(S - run) * N * sizeof(float2)}};
+  BCK(b->host_stage.download(parts, 2, true, b->device, b->st));
   return FELIS_OK;
 }
 

@@ -58,6 +58,26 @@ __global__ void k_f32_to_bf16(const float* in, bf16* out, int64_t n) {
     out[i] = __float2bfloat16_rn(in[i]);
 }
 
+__global__ void k_pack_rows(const float* __restrict__ in, int rows, int cols, int rows_pad, int cols_pad,
+                            __nv_bfloat162* __restrict__ out) {
+  const int half = cols_pad >> 1;
+  const int64_t n = (int64_t)rows_pad * half;
+  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
+    const int r = (int)(i / half), c = 2 * (int)(i - (int64_t)r * half);
+    const float* p = in + (size_t)r * cols + c;
+    const float a = r < rows && c < cols ? p[0] : 0.f, b = r < rows && c + 1 < cols ? p[1] : 0.f;
+    out[i] = __floats2bfloat162_rn(a, b);
+  }
+}
+
+__global__ void k_unpad_rows(const float* __restrict__ in, int rows, int ld, int cols, float* __restrict__ out) {
+  const int64_t n = (int64_t)rows * cols;
+  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
+    const int r = (int)(i / cols);
+    out[i] = in[(size_t)r * ld + (i - (int64_t)r * cols)];
+  }
+}
+
 __global__ void k_transpose_bf16(const bf16* in, int rows, int cols, int ld_in, bf16* out, int rows_pad,
                                  int cols_pad) {
   const int64_t n = (int64_t)rows_pad * cols_pad;
@@ -130,6 +150,16 @@ int grid_for(int64_t n) { return (int)((n + 255) / 256 < 4096 ? (n + 255) / 256 
 
 void launch_f32_to_bf16(const float* in, bf16* out, int64_t n, cudaStream_t st) {
   if (n > 0) k_f32_to_bf16<<<grid_for(n), 256, 0, st>>>(in, out, n);
+}
+
+void launch_pack_rows(const float* in, int rows, int cols, int rows_pad, int cols_pad, bf16* out, cudaStream_t st) {
+  const int64_t n = (int64_t)rows_pad * (cols_pad >> 1);
+  if (n > 0) k_pack_rows<<<grid_for(n), 256, 0, st>>>(in, rows, cols, rows_pad, cols_pad, reinterpret_cast<__nv_bfloat162*>(out));
+}
+
+void launch_unpad_rows(const float* in, int rows, int ld, int cols, float* out, cudaStream_t st) {
+  const int64_t n = (int64_t)rows * cols;
+  if (n > 0) k_unpad_rows<<<grid_for(n), 256, 0, st>>>(in, rows, ld, cols, out);
 }
 
 void launch_transpose_bf16(const bf16* in, int rows, int cols, int ld_in, bf16* out, int rows_pad, int cols_pad,

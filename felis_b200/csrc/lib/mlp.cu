@@ -17,6 +17,7 @@
 
 #include "../../../include/felis_b200.h"
 #include "mlp.cuh"
+#include "transfer.cuh"
 
 using namespace felis;
 
@@ -67,6 +68,8 @@ struct felis_mlp {
   float* dt = nullptr;
   int64_t n_data = 0;
   int* d_idx = nullptr;
+  int device = 0;
+  HostStage stage;  // rows of inference calls
 };
 
 namespace {
@@ -288,6 +291,7 @@ felis_status felis_mlp_create(int32_t n_in, int32_t width, int32_t n_out, uint64
     felis_mlp_destroy(m);
     return s;
   };
+  cudaGetDevice(&m->device);
   cudaError_t e = cudaStreamCreateWithFlags(&m->st, cudaStreamNonBlocking);
   if (e == cudaSuccess) e = cudaMalloc(&m->d_err, sizeof(int));
   if (e == cudaSuccess) e = cudaMemset(m->d_err, 0, sizeof(int));
@@ -380,22 +384,23 @@ felis_status felis_mlp_forward(felis_mlp* m, const float* x, int64_t n, float* y
   felis_status s =
       ensure_cap(m, (int)std::min<int64_t>(round_up((int)std::min<int64_t>(n, kFwdChunk), 128), kFwdChunk));
   if (s != FELIS_OK) return s;
-  std::vector<float> hy;
   for (int64_t r0 = 0; r0 < n; r0 += kFwdChunk) {
     const int nr = (int)std::min<int64_t>(kFwdChunk, n - r0);
     const int M = round_up(nr, 128);
-    MCK(cudaMemsetAsync(m->xf, 0, (size_t)M * m->in_p * sizeof(float), m->st));
-    s = upload_rows(m, x + (size_t)r0 * m->n_in, nr, m->n_in, m->in_p, m->xf);
-    if (s != FELIS_OK) return s;
-    launch_f32_to_bf16(m->xf, m->xb, (int64_t)M * m->in_p, m->st);
+    // the rows cross the link as they are, in and out; padding and rounding
+    // are done on the device
+    const CopyPart in{x + (size_t)r0 * m->n_in, m->xf, (size_t)nr * m->n_in * sizeof(float)};
+    MCK(m->stage.upload(&in, 1, m->device, m->st));
+    launch_pack_rows(m->xf, nr, m->n_in, M, m->in_p, m->xb, m->st);
     MCK(cudaEventRecord(m->ev0, m->st));
     if (m->fused) forward_fused(m, M);
     else forward(m, M, false);
     MCK(cudaEventRecord(m->ev1, m->st));
-    hy.resize((size_t)nr * m->out_p);
-    MCK(cudaMemcpyAsync(hy.data(), m->z[kLayers - 1], hy.size() * sizeof(float), cudaMemcpyDeviceToHost, m->st));
+    launch_unpad_rows(m->z[kLayers - 1], nr, m->out_p, m->n_out, m->xf, m->st);
+    MCK(cudaGetLastError());
+    const CopyPart out{m->xf, y + (size_t)r0 * m->n_out, (size_t)nr * m->n_out * sizeof(float)};
+    MCK(m->stage.download(&out, 1, false, m->device, m->st));
     MCK(cudaStreamSynchronize(m->st));
-    for (int r = 0; r < nr; ++r) memcpy(y + (size_t)(r0 + r) * m->n_out, &hy[(size_t)r * m->out_p], m->n_out * sizeof(float));
     float ms = 0.f;
     MCK(cudaEventElapsedTime(&ms, m->ev0, m->ev1));
     m->fwd_ms = ms;

@@ -64,6 +64,11 @@ cudaError_t launch_mlp_fused(const MlpFusedArgs& a, cudaStream_t st);
 
 // Elementwise and reduction helpers (row-major [rows][cols] unless stated).
 void launch_f32_to_bf16(const float* in, bf16* out, int64_t n, cudaStream_t st);
+// out[r][c] = in[r][c] in BF16, rows x cols of a dense matrix into a padded one
+// of rows_pad x cols_pad (cols_pad even), zeros around them
+void launch_pack_rows(const float* in, int rows, int cols, int rows_pad, int cols_pad, bf16* out, cudaStream_t st);
+// out[r][c] = in[r][c], the first cols of ld columns, densely packed
+void launch_unpad_rows(const float* in, int rows, int ld, int cols, float* out, cudaStream_t st);
 // out[c][r] = in[r][c] for r < rows, c < cols; rows_pad / cols_pad zero padding
 // of the destination ([cols_pad][rows_pad])
 void launch_transpose_bf16(const bf16* in, int rows, int cols, int ld_in, bf16* out, int rows_pad, int cols_pad,

@@ -1,0 +1,40 @@
+// Large copies between the device and pageable host memory.
+#pragma once
+
+#include <cuda_runtime.h>
+#include <stddef.h>
+
+namespace felis {
+
+struct CopyPart {
+  const void* src;
+  void* dst;
+  size_t bytes;  // at the source (a multiple of 4)
+};
+
+// Page-locked slots of one handle, ensemble or network, made at its first copy
+// and freed with it (16 MB at most).  One call at a time, like its owner.
+class HostStage {
+ public:
+  HostStage() = default;
+  HostStage(const HostStage&) = delete;
+  HostStage& operator=(const HostStage&) = delete;
+  ~HostStage();
+  // Copies every part to the host, FP32 values widened to FP64 when `widen`
+  // (the destination then holds twice the bytes).  Returns when all is there.
+  cudaError_t download(const CopyPart* parts, int nparts, bool widen, int device, cudaStream_t st);
+  // Copies every part to the device.  Returns when all is there.
+  cudaError_t upload(const CopyPart* parts, int nparts, int device, cudaStream_t st);
+
+ private:
+  static constexpr int kThreads = 8, kSlots = 2;
+  static constexpr size_t kChunk = (size_t)1 << 20;
+  char* pinned_ = nullptr;  // [threads_][kSlots][kChunk]
+  cudaEvent_t ev_[kThreads][kSlots] = {};
+  int threads_ = 0;
+  cudaError_t reserve(int threads);
+  enum Mode { kDown, kDownWiden, kUp };
+  cudaError_t run(const CopyPart* parts, int nparts, Mode mode, int device, cudaStream_t st);
+};
+
+}  // namespace felis
