@@ -1,9 +1,14 @@
 // BF16 GEMM of the taper surrogate on the 5th-generation tensor cores:
 // C[M][N] = A[M][K] . B[N][K]^T, FP32 accumulation in tensor memory, with the
-// epilogue of mlp.cuh (bias, GELU, FP32 and/or BF16 outputs).
+// epilogue of mlp.cuh (bias, GELU or its derivative, FP32 and/or BF16 outputs,
+// a transposed copy for the next GEMM that contracts over the rows).
 //
-// One persistent CTA per SM walks the 128-row tiles of C (N <= 256 columns,
-// one tile wide).  Warp roles:
+// One launch computes one or two independent products (the weight gradient of
+// a layer and the gradient of its input, which use the same dz): one
+// persistent CTA per SM walks the tiles of both, 128 rows by up to 256
+// columns.  A training batch has a handful of rows of tiles, and a 256-column
+// epilogue (GELU, two or three outputs) takes its SM 15 us, so small products
+// are cut into narrower tiles until they cover the SMs.  Warp roles:
 //   warp 0     one lane issues the TMA loads: the A tile (128 x 64) and the
 //              B tile (N x 64) of every 64-column K chunk, 128-byte swizzle,
 //              into a ring of kStages shared-memory stages (full / empty
@@ -43,18 +48,26 @@ constexpr int kThreads = 32 * (2 + kEpiWarps);
 constexpr uint32_t kABytes = kBM * kBK * 2;  // 16 KB
 
 struct TmaGemm {
-  int M, N, K;     // M a multiple of 128, N a multiple of 16 (<= 256), K a multiple of 16
-  int tmem_cols;   // allocated tensor-memory columns
-  int acc_stride;  // column offset of the second accumulator (N rounded up to 32)
+  int M, N, K;  // M a multiple of 128, N a multiple of 16 (<= 256), K a multiple of 16
   const float* bias;
+  const float* z;  // multiply by GELU'(z)
   float* out_f32;
   bf16* out_bf16;
-  int ldc, n_valid, gelu;
+  bf16* out_t;
+  int ldc, ldt, n_valid, gelu;
+  int bn, nt;  // columns of a tile, tiles per 128 rows
+};
+struct TmaPair {
+  TmaGemm g[2];
+  CUtensorMap a[2], b[2];
+  int tiles0, tiles;     // tiles of the first product, of both
+  int tmem_cols;         // allocated tensor-memory columns
+  int acc_stride;        // column offset of the second accumulator (the wider tile rounded up to 32)
+  uint32_t stage_bytes;  // of the wider tile
   int* err;
 };
 
-__global__ void __launch_bounds__(kThreads, 1) k_gemm_tma(const __grid_constant__ CUtensorMap tmA,
-                                                           const __grid_constant__ CUtensorMap tmB, TmaGemm g) {
+__global__ void __launch_bounds__(kThreads, 1) k_gemm_tma(const __grid_constant__ TmaPair P) {
   extern __shared__ unsigned char smraw[];
   __shared__ __align__(8) uint64_t full[kStages], empty[kStages], tfull[2], tempty[2];
   __shared__ uint32_t tmem_slot;
@@ -62,10 +75,8 @@ __global__ void __launch_bounds__(kThreads, 1) k_gemm_tma(const __grid_constant_
   // the swizzled operand tiles start on 1024-byte boundaries of the shared window
   unsigned char* sm = smraw + ((1024u - (sa(smraw) & 1023u)) & 1023u);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int N = g.N;
-  const uint32_t stage_bytes = kABytes + (uint32_t)N * kBK * 2;
-  const int ntiles = g.M / kBM;
-  const int nk = (g.K + kBK - 1) / kBK;
+  const uint32_t stage_bytes = P.stage_bytes;
+  const int ntiles = P.tiles;
   volatile int* abort_v = &abort_flag;
 
   if (threadIdx.x == 0) {
@@ -82,7 +93,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_gemm_tma(const __grid_constant_
   }
   if (warp == 1) {
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;\n" ::"r"(sa(&tmem_slot)),
-                 "r"(g.tmem_cols)
+                 "r"(P.tmem_cols)
                  : "memory");
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;\n" ::: "memory");
   }
@@ -93,31 +104,33 @@ __global__ void __launch_bounds__(kThreads, 1) k_gemm_tma(const __grid_constant_
 
   auto give_up = [&]() {
     *abort_v = 1;
-    if (g.err) atomicOr(g.err, 1);
+    if (P.err) atomicOr(P.err, 1);
   };
 
   if (warp == 0) {
     if (lane == 0) {
-      asm volatile("prefetch.tensormap [%0];\n" ::"l"(reinterpret_cast<uint64_t>(&tmA)) : "memory");
-      asm volatile("prefetch.tensormap [%0];\n" ::"l"(reinterpret_cast<uint64_t>(&tmB)) : "memory");
       int s = 0;
       uint32_t ph = 0;
       bool ok = true;
-      for (int t = blockIdx.x; t < ntiles && ok; t += gridDim.x)
+      for (int t = blockIdx.x; t < ntiles && ok; t += gridDim.x) {
+        const int p = t >= P.tiles0, tp = p ? t - P.tiles0 : t, m = tp / P.g[p].nt * kBM;
+        const int n0 = tp % P.g[p].nt * P.g[p].bn;
+        const int nk = (P.g[p].K + kBK - 1) / kBK;
+        const uint32_t bytes = kABytes + (uint32_t)P.g[p].bn * kBK * 2;
         for (int k = 0; k < nk && ok; ++k) {
           // a fresh stage passes at once (the phase before the first counts as complete)
           if (!mbar_wait(sa(&empty[s]), ph ^ 1u, abort_v)) { give_up(); ok = false; break; }
           const uint32_t a_s = sa(sm + (size_t)s * stage_bytes);
-          mbar_expect_tx(sa(&full[s]), stage_bytes);
-          tma_load_2d(a_s, &tmA, k * kBK, t * kBM, sa(&full[s]));
-          tma_load_2d(a_s + kABytes, &tmB, k * kBK, 0, sa(&full[s]));
+          mbar_expect_tx(sa(&full[s]), bytes);
+          tma_load_2d(a_s, &P.a[p], k * kBK, m, sa(&full[s]));
+          tma_load_2d(a_s + kABytes, &P.b[p], k * kBK, n0, sa(&full[s]));
           if (++s == kStages) { s = 0; ph ^= 1u; }
         }
+      }
     }
     __syncwarp();
   } else if (warp == 1) {
     if (lane == 0) {
-      const uint32_t idesc = idesc_bf16(kBM, N);
       int s = 0, it = 0;
       uint32_t ph = 0;
       uint32_t last_bar = 0, last_par = 0;  // last commit, waited for on the way out
@@ -127,7 +140,10 @@ __global__ void __launch_bounds__(kThreads, 1) k_gemm_tma(const __grid_constant_
         const uint32_t bph = (uint32_t)(it >> 1) & 1u;
         if (!mbar_wait(sa(&tempty[b]), bph ^ 1u, abort_v)) { give_up(); ok = false; break; }
         asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
-        const uint32_t d = tmem + (uint32_t)(b * g.acc_stride);
+        const uint32_t d = tmem + (uint32_t)(b * P.acc_stride);
+        const TmaGemm& g = P.g[t >= P.tiles0];
+        const uint32_t idesc = idesc_bf16(kBM, g.bn);
+        const int nk = (g.K + kBK - 1) / kBK;
         for (int k = 0; k < nk; ++k) {
           if (!mbar_wait(sa(&full[s]), ph, abort_v)) { give_up(); ok = false; break; }
           asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
@@ -161,11 +177,16 @@ __global__ void __launch_bounds__(kThreads, 1) k_gemm_tma(const __grid_constant_
       const uint32_t bph = (uint32_t)(it >> 1) & 1u;
       if (!mbar_wait(sa(&tfull[b]), bph, abort_v)) { give_up(); break; }
       asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
-      const uint32_t tbase = tmem + ((uint32_t)(q * 32) << 16) + (uint32_t)(b * g.acc_stride);
-      const size_t row = (size_t)t * kBM + (size_t)q * 32 + lane;
-      for (int c0 = 32 * half; c0 < N; c0 += 64) {
+      const uint32_t tbase = tmem + ((uint32_t)(q * 32) << 16) + (uint32_t)(b * P.acc_stride);
+      const int p = t >= P.tiles0;
+      const TmaGemm& g = P.g[p];
+      const int tp = p ? t - P.tiles0 : t, n0 = tp % g.nt * g.bn;
+      const int N = min(g.N, n0 + g.bn);
+      const size_t row = (size_t)(tp / g.nt) * kBM + (size_t)q * 32 + lane;
+#pragma unroll 1
+      for (int c0 = n0 + 32 * half; c0 < N; c0 += 64) {
         uint32_t r[32];
-        TMEM_LD32X32(tbase + (uint32_t)c0, r);
+        TMEM_LD32X32(tbase + (uint32_t)(c0 - n0), r);
         asm volatile("tcgen05.wait::ld.sync.aligned;\n" ::: "memory");
         const int ncol = N - c0 < 32 ? N - c0 : 32;  // 16 or 32 (N is a multiple of 16)
         float v[32];
@@ -182,23 +203,42 @@ __global__ void __launch_bounds__(kThreads, 1) k_gemm_tma(const __grid_constant_
           for (int j = 0; j < 8; ++j)
             if (4 * j < ncol) dst[j] = make_float4(v[4 * j], v[4 * j + 1], v[4 * j + 2], v[4 * j + 3]);
         }
-        if (g.out_bf16) {
-          uint4* dst = reinterpret_cast<uint4*>(g.out_bf16 + o);
+        if (g.z) {
+          const float4* zs = reinterpret_cast<const float4*>(g.z + o);
 #pragma unroll
-          for (int j = 0; j < 4; ++j) {
-            if (8 * j >= ncol) break;
-            uint32_t w[4];
-#pragma unroll
-            for (int k = 0; k < 4; ++k) {
-              float x0 = v[8 * j + 2 * k], x1 = v[8 * j + 2 * k + 1];
-              if (g.gelu) {
-                if (c0 + 8 * j + 2 * k < g.n_valid) x0 = gelu_f(x0);
-                if (c0 + 8 * j + 2 * k + 1 < g.n_valid) x1 = gelu_f(x1);
-              }
-              const __nv_bfloat162 p2 = __floats2bfloat162_rn(x0, x1);
-              w[k] = *reinterpret_cast<const uint32_t*>(&p2);
+          for (int j = 0; j < 8; ++j)
+            if (4 * j < ncol) {
+              const float4 z = zs[j];
+              v[4 * j] *= gelu_grad(z.x);
+              v[4 * j + 1] *= gelu_grad(z.y);
+              v[4 * j + 2] *= gelu_grad(z.z);
+              v[4 * j + 3] *= gelu_grad(z.w);
             }
-            dst[j] = make_uint4(w[0], w[1], w[2], w[3]);
+        }
+        if (g.out_bf16 || g.out_t) {
+          uint32_t w[16];
+#pragma unroll
+          for (int k = 0; k < 16; ++k) {
+            float x0 = v[2 * k], x1 = v[2 * k + 1];
+            if (g.gelu) {
+              if (c0 + 2 * k < g.n_valid) x0 = gelu_f(x0);
+              if (c0 + 2 * k + 1 < g.n_valid) x1 = gelu_f(x1);
+            }
+            const __nv_bfloat162 p2 = __floats2bfloat162_rn(x0, x1);
+            w[k] = *reinterpret_cast<const uint32_t*>(&p2);
+          }
+          if (g.out_bf16) {
+            uint4* dst = reinterpret_cast<uint4*>(g.out_bf16 + o);
+#pragma unroll
+            for (int j = 0; j < 4; ++j)
+              if (8 * j < ncol) dst[j] = make_uint4(w[4 * j], w[4 * j + 1], w[4 * j + 2], w[4 * j + 3]);
+          }
+          if (g.out_t) {
+            // 32 neighbouring rows of one column by a warp: 64 bytes
+            uint16_t* dst = reinterpret_cast<uint16_t*>(g.out_t) + (size_t)c0 * g.ldt + row;
+#pragma unroll
+            for (int j = 0; j < 32; ++j)
+              if (j < ncol) dst[(size_t)j * g.ldt] = (uint16_t)(w[j >> 1] >> (16 * (j & 1)));
           }
         }
       }
@@ -209,7 +249,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_gemm_tma(const __grid_constant_
   asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
   __syncthreads();
   if (warp == 1)
-    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;\n" ::"r"(tmem), "r"(g.tmem_cols) : "memory");
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;\n" ::"r"(tmem), "r"(P.tmem_cols) : "memory");
 }
 
 typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*,
@@ -252,26 +292,45 @@ cudaError_t gemm_tma_prepare() {
   return e;
 }
 
-cudaError_t launch_gemm_tma(const GemmArgs& a, cudaStream_t st) {
+cudaError_t launch_gemm_tma(const GemmArgs* a, int n, cudaStream_t st) {
   if (!g_encode || g_sms <= 0) return cudaErrorNotReady;
-  if (a.M % kBM || a.N % 16 || a.N < 16 || a.N > 256 || a.K % 16 || a.K < 16 || a.lda % 8 || a.ldb % 8 ||
-      (reinterpret_cast<uintptr_t>(a.A) & 15) || (reinterpret_cast<uintptr_t>(a.B) & 15))
-    return cudaErrorInvalidValue;
-  CUtensorMap ta, tb;
-  if (!tma_encode_bf16(&ta, a.A, a.M, a.K, a.lda, kBM) || !tma_encode_bf16(&tb, a.B, a.N, a.K, a.ldb, a.N)) return cudaErrorInvalidValue;
-  TmaGemm g;
-  g.M = a.M; g.N = a.N; g.K = a.K;
+  if (n < 1 || n > 2) return cudaErrorInvalidValue;
+  TmaPair P{};
+  int wide = 0;
+  for (int i = 0; i < n; ++i) {
+    const GemmArgs& x = a[i];
+    if (x.M % kBM || x.N % 16 || x.N < 16 || x.N > 256 || x.K % 16 || x.K < 16 || x.lda % 8 || x.ldb % 8 ||
+        (reinterpret_cast<uintptr_t>(x.A) & 15) || (reinterpret_cast<uintptr_t>(x.B) & 15))
+      return cudaErrorInvalidValue;
+    // rows of A past rows_a read as zero
+    const int rows_a = x.rows_a ? x.rows_a : x.M;
+    TmaGemm& g = P.g[i];
+    // tiles as wide as the product while the launch fills the SMs, else 64 or
+    // 32 columns (rows of B past N count as zero).  512 x 256 with GELU and
+    // both outputs: 31 us as four tiles of 256 columns, 10.3 us as 32 of 32
+    g.bn = x.N;
+    for (int bn : {64, 32})
+      if (g.bn > bn && (x.M / kBM) * ((x.N + g.bn - 1) / g.bn) * 2 <= g_sms) g.bn = bn;
+    g.nt = (x.N + g.bn - 1) / g.bn;
+    if (!tma_encode_bf16(&P.a[i], x.A, rows_a, x.K, x.lda, kBM) || !tma_encode_bf16(&P.b[i], x.B, x.N, x.K, x.ldb, g.bn))
+      return cudaErrorInvalidValue;
+    g.M = x.M; g.N = x.N; g.K = x.K;
+    g.bias = x.bias; g.z = x.z; g.out_f32 = x.out_f32; g.out_bf16 = x.out_bf16; g.out_t = x.out_t;
+    g.ldc = x.ldc; g.ldt = x.ldt; g.n_valid = x.n_valid; g.gelu = x.gelu;
+    P.tiles += x.M / kBM * g.nt;
+    if (i == 0) P.tiles0 = P.tiles;
+    if (g.bn > wide) wide = g.bn;
+  }
   // two accumulators 32-column aligned (the epilogue reads 32 columns at a
   // time), in a power-of-two allocation of at least 32 columns
-  g.acc_stride = (a.N + 31) & ~31;
-  int cols = 32;
-  while (cols < 2 * g.acc_stride) cols <<= 1;
-  g.tmem_cols = cols;
-  g.bias = a.bias; g.out_f32 = a.out_f32; g.out_bf16 = a.out_bf16;
-  g.ldc = a.ldc; g.n_valid = a.n_valid; g.gelu = a.gelu; g.err = a.err;
-  const int tiles = a.M / kBM;
-  const int grid = tiles < g_sms ? tiles : g_sms;
-  k_gemm_tma<<<grid, kThreads, tma_smem(a.N), st>>>(ta, tb, g);
+  P.acc_stride = (wide + 31) & ~31;
+  P.tmem_cols = 32;
+  while (P.tmem_cols < 2 * P.acc_stride) P.tmem_cols <<= 1;
+  P.stage_bytes = kABytes + (uint32_t)wide * kBK * 2;
+  P.err = a[0].err;
+  const int grid = P.tiles < g_sms ? P.tiles : g_sms;
+  if (grid == 0) return cudaSuccess;
+  k_gemm_tma<<<grid, kThreads, tma_smem(wide), st>>>(P);
   return cudaGetLastError();
 }
 

@@ -51,25 +51,26 @@ struct felis_mlp {
   bf16* wt[kLayers] = {};    // BF16 transposed weights [cols][rows] (layers 2..4)
   int64_t steps = 0;
   // activations of one chunk
-  int cap = 0;
+  int cap = 0, layer_cap = 0, train_cap = 0;
+  char* layer_buf = nullptr;  // holds tgt and the hidden layers' z and a
+  bf16* train_buf = nullptr;  // holds dz, dzt and at
   bf16* xb = nullptr;        // [cap][in_p]
   float* xf = nullptr;       // staging for uploads [cap][max(in_p, out_p)]
   float* z[kLayers] = {};    // pre-activations [cap][rows]
-  bf16* a[kLayers] = {};     // activations / outputs [cap][rows]
+  bf16* a[kLayers] = {};     // hidden activations [cap][rows]
   float* tgt = nullptr;      // targets [cap][out_p]
-  bf16* dz = nullptr;        // [cap][width]
-  bf16* dzt = nullptr;       // transposed [max(width, out_rows)][cap]
-  bf16* at = nullptr;        // transposed activation [max(width, in_p)][cap]
-  float* da = nullptr;       // [cap][width]
+  bf16* dz[kLayers] = {};    // [cap][rows]
+  bf16* dzt[kLayers] = {};   // transposed [rows][batch rows]
+  bf16* at[kLayers] = {};    // transposed inputs of the layers [cols][batch rows]
   double* loss_part = nullptr;
-  std::vector<double> h_part;
+  int64_t loss_cap = 0;
   // training set
   bf16* dx = nullptr;
   float* dt = nullptr;
   int64_t n_data = 0;
   int* d_idx = nullptr;
   int device = 0;
-  HostStage stage;  // rows of inference calls
+  HostStage stage;  // rows of inference and gradient calls
 };
 
 namespace {
@@ -88,20 +89,6 @@ felis_status mfail(felis_mlp* m, felis_status s, const std::string& e) {
   return s;
 }
 
-__global__ void k_gather_rows(const bf16* x, const float* t, const int* idx, int n, int in_p, int out_p, bf16* xb,
-                              float* tb) {
-  const int r = blockIdx.x;
-  if (r >= n) return;
-  const int64_t s = idx[r];
-  for (int c = threadIdx.x; c < in_p; c += blockDim.x) xb[(size_t)r * in_p + c] = x[s * in_p + c];
-  for (int c = threadIdx.x; c < out_p; c += blockDim.x) tb[(size_t)r * out_p + c] = t[s * out_p + c];
-}
-
-__global__ void k_zero_rows_bf16(bf16* x, int64_t from, int64_t to) {
-  for (int64_t i = from + blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < to; i += (int64_t)gridDim.x * blockDim.x)
-    x[i] = __float2bfloat16_rn(0.f);
-}
-
 // Host rows [n][c_real] (FP32) -> device padded rows [n][c_pad].
 felis_status upload_rows(felis_mlp* m, const float* h, int64_t n, int c_real, int c_pad, float* d) {
   std::vector<float> buf((size_t)n * c_pad, 0.f);
@@ -111,39 +98,72 @@ felis_status upload_rows(felis_mlp* m, const float* h, int64_t n, int c_real, in
   return FELIS_OK;
 }
 
-felis_status ensure_cap(felis_mlp* m, int rows) {
-  if (rows <= m->cap) return FELIS_OK;
-  void** bufs[] = {(void**)&m->xb, (void**)&m->xf, (void**)&m->tgt, (void**)&m->dz, (void**)&m->dzt,
-                   (void**)&m->at, (void**)&m->da, (void**)&m->loss_part};
-  for (auto b : bufs) { if (*b) cudaFree(*b); *b = nullptr; }
-  for (int l = 0; l < kLayers; ++l) {
-    if (m->z[l]) cudaFree(m->z[l]);
-    if (m->a[l]) cudaFree(m->a[l]);
-    m->z[l] = nullptr;
-    m->a[l] = nullptr;
+// Buffers of an inference pass over `rows` rows; the hidden layers' and the
+// targets' only where `layers` (the fused kernel keeps them on chip).
+felis_status ensure_cap(felis_mlp* m, int rows, bool layers) {
+  if (rows > m->cap) {
+    void** bufs[] = {(void**)&m->xb, (void**)&m->xf, (void**)&m->z[kLayers - 1]};
+    for (auto b : bufs) { if (*b) cudaFree(*b); *b = nullptr; }
+    m->cap = 0;
+    MCK(cudaMalloc(&m->xb, (size_t)rows * m->in_p * sizeof(bf16)));
+    MCK(cudaMalloc(&m->xf, (size_t)rows * std::max(m->in_p, m->out_p) * sizeof(float)));
+    MCK(cudaMalloc(&m->z[kLayers - 1], (size_t)rows * m->out_p * sizeof(float)));
+    m->cap = rows;
   }
-  m->cap = rows;
-  const int wide = std::max(m->width, std::max(m->in_p, m->out_rows));
-  MCK(cudaMalloc(&m->xb, (size_t)rows * m->in_p * sizeof(bf16)));
-  MCK(cudaMalloc(&m->xf, (size_t)rows * std::max(m->in_p, m->out_p) * sizeof(float)));
-  MCK(cudaMalloc(&m->tgt, (size_t)rows * m->out_p * sizeof(float)));
-  MCK(cudaMalloc(&m->dz, (size_t)rows * m->width * sizeof(bf16)));
-  MCK(cudaMalloc(&m->dzt, (size_t)wide * rows * sizeof(bf16)));
-  MCK(cudaMalloc(&m->at, (size_t)wide * rows * sizeof(bf16)));
-  MCK(cudaMalloc(&m->da, (size_t)rows * m->width * sizeof(float)));
-  MCK(cudaMalloc(&m->loss_part, (size_t)mse_blocks(rows) * sizeof(double)));
-  for (int l = 0; l < kLayers; ++l) {
-    MCK(cudaMalloc(&m->z[l], (size_t)rows * m->rows[l] * sizeof(float)));
-    MCK(cudaMalloc(&m->a[l], (size_t)rows * m->rows[l] * sizeof(bf16)));
+  if (layers && rows > m->layer_cap) {
+    // one allocation: every part is a multiple of 128 rows by 16 columns
+    if (m->layer_buf) cudaFree(m->layer_buf);
+    m->layer_buf = nullptr;
+    m->layer_cap = 0;
+    size_t bytes = (size_t)rows * m->out_p * sizeof(float);
+    for (int l = 0; l < kLayers - 1; ++l) bytes += (size_t)rows * m->rows[l] * (sizeof(float) + sizeof(bf16));
+    MCK(cudaMalloc(&m->layer_buf, bytes));
+    char* at = m->layer_buf;
+    auto take = [&](size_t n) { char* q = at; at += n; return q; };
+    m->tgt = (float*)take((size_t)rows * m->out_p * sizeof(float));
+    for (int l = 0; l < kLayers - 1; ++l) {
+      m->z[l] = (float*)take((size_t)rows * m->rows[l] * sizeof(float));
+      m->a[l] = (bf16*)take((size_t)rows * m->rows[l] * sizeof(bf16));
+    }
+    m->layer_cap = rows;
   }
-  m->h_part.assign(mse_blocks(rows), 0.0);
   return FELIS_OK;
 }
 
-void gemm(felis_mlp* m, const bf16* A, const bf16* B, int M, int N, int K, int lda, int ldb, const float* bias,
-          float* out_f32, bf16* out_bf16, int ldc, int n_valid, int gelu) {
-  GemmArgs g{A, B, M, N, K, lda, ldb, bias, out_f32, out_bf16, ldc, n_valid, gelu, m->d_err};
-  if (launch_gemm_tma(g, m->st) != cudaSuccess) {
+// What training needs besides: dz and the transposed operands of `rows` rows,
+// and `parts` partial losses.
+felis_status ensure_train(felis_mlp* m, int rows, int64_t parts) {
+  felis_status s = ensure_cap(m, rows, true);
+  if (s != FELIS_OK) return s;
+  if (rows > m->train_cap) {
+    if (m->train_buf) cudaFree(m->train_buf);
+    m->train_buf = nullptr;
+    m->train_cap = 0;
+    size_t n = 0;
+    for (int l = 0; l < kLayers; ++l) n += (size_t)rows * (2 * m->rows[l] + m->cols[l]);
+    MCK(cudaMalloc(&m->train_buf, n * sizeof(bf16)));
+    bf16* at = m->train_buf;
+    auto take = [&](size_t k) { bf16* q = at; at += k; return q; };
+    for (int l = 0; l < kLayers; ++l) {
+      m->dz[l] = take((size_t)rows * m->rows[l]);
+      m->dzt[l] = take((size_t)rows * m->rows[l]);
+      m->at[l] = take((size_t)rows * m->cols[l]);
+    }
+    m->train_cap = rows;
+  }
+  if (parts > m->loss_cap) {
+    if (m->loss_part) cudaFree(m->loss_part);
+    m->loss_part = nullptr;
+    m->loss_cap = 0;
+    MCK(cudaMalloc(&m->loss_part, (size_t)parts * sizeof(double)));
+    m->loss_cap = parts;
+  }
+  return FELIS_OK;
+}
+
+// One product, or two independent ones, in a launch.
+void gemm(felis_mlp* m, const GemmArgs* g, int n) {
+  if (launch_gemm_tma(g, n, m->st) != cudaSuccess) {
     // shapes the network never produces (M % 128, N > 256, unaligned rows):
     // reported through the error word like a device failure
     cudaMemsetAsync(m->d_err, 0xff, sizeof(int), m->st);
@@ -151,17 +171,22 @@ void gemm(felis_mlp* m, const bf16* A, const bf16* B, int M, int N, int K, int l
 }
 
 // Forward pass of rows [0, M) of xb (M a multiple of 128).  Training keeps
-// every layer's FP32 pre-activation z (the backward pass needs it);
-// inference writes the hidden layers' BF16 activations and the last layer's
-// FP32 output only.
-void forward(felis_mlp* m, int M, bool keep_z = true) {
+// every layer's FP32 pre-activation z (the backward pass needs it) and the
+// hidden activations both ways round; inference writes the hidden layers' BF16
+// activations and the last layer's FP32 output only.
+void forward(felis_mlp* m, int M, bool train = true) {
   const bf16* in = m->xb;
   int ld_in = m->in_p;
   for (int l = 0; l < kLayers; ++l) {
     const bool last = l == kLayers - 1;
-    gemm(m, in, m->wb[l], M, m->rows[l], m->cols[l], ld_in, m->cols[l], m->p + m->b_off[l],
-         (keep_z || last) ? m->z[l] : nullptr, (keep_z || !last) ? m->a[l] : nullptr,
-         m->rows[l], m->rows_real[l], last ? 0 : 1);
+    GemmArgs g{in, m->wb[l], M, m->rows[l], m->cols[l], ld_in, m->cols[l], m->p + m->b_off[l],
+               (train || last) ? m->z[l] : nullptr, last ? nullptr : m->a[l],
+               m->rows[l], m->rows_real[l], last ? 0 : 1, m->d_err};
+    if (train && !last) {
+      g.out_t = m->at[l + 1];
+      g.ldt = M;
+    }
+    gemm(m, &g, 1);
     in = m->a[l];
     ld_in = m->rows[l];
   }
@@ -182,34 +207,40 @@ void forward_fused(felis_mlp* m, int M) {
   if (launch_mlp_fused(a, m->st) != cudaSuccess) cudaMemsetAsync(m->d_err, 0xff, sizeof(int), m->st);
 }
 
+MlpLayers layers_of(const felis_mlp* m) {
+  MlpLayers L{};
+  for (int l = 0; l < kLayers; ++l) {
+    L.w_off[l] = m->w_off[l]; L.b_off[l] = m->b_off[l];
+    L.rows[l] = m->rows[l]; L.cols[l] = m->cols[l];
+    L.wb[l] = m->wb[l]; L.wt[l] = m->wt[l]; L.dzt[l] = m->dzt[l];
+  }
+  return L;
+}
+
 // Gradients of the mean squared error over the first n_real rows of the
-// chunk (targets in tgt) into m->grad; returns the summed squared error.
-felis_status backward(felis_mlp* m, int M, int n_real, double* sse) {
+// chunk (targets in tgt, inputs both ways round in xb and at[0]) into m->grad;
+// the squared errors' block sums go to loss_part.
+void backward(felis_mlp* m, int M, int n_real, double* loss_part) {
   const int L = kLayers;
   const float scale = 2.f / ((float)n_real * (float)m->n_out);
-  launch_mse_grad(m->z[L - 1], m->tgt, M, n_real, m->out_p, m->n_out, scale, m->dz, m->loss_part, m->st);
-  int dz_cols = m->out_p;  // current dz is [M][dz_cols]
+  launch_mse_grad(m->z[L - 1], m->tgt, M, n_real, m->out_p, m->n_out, scale, m->dz[L - 1], m->dzt[L - 1], loss_part, m->st);
   for (int l = L - 1; l >= 0; --l) {
     const int R = m->rows[l], Cc = m->cols[l];
-    const int Rt = l == L - 1 ? m->out_rows : R;  // transposed dz rows (A operand: a multiple of 128)
-    // dW = dz^T . a_{l-1}: A = dz^T [Rt][M], B = a_{l-1}^T [Cc][M]
-    launch_transpose_bf16(m->dz, M, dz_cols, dz_cols, m->dzt, M, Rt, m->st);
-    const bf16* prev = l == 0 ? m->xb : m->a[l - 1];
-    launch_transpose_bf16(prev, M, Cc, Cc, m->at, M, Cc, m->st);
-    gemm(m, m->dzt, m->at, Rt, Cc, M, M, M, nullptr, m->grad + m->w_off[l], nullptr, Cc, Cc, 0);
-    launch_col_sum(m->dz, M, dz_cols, m->grad + m->b_off[l], m->st);
-    if (l == 0) break;
-    // da_{l-1} = dz . W_l: A = dz [M][R], B = W_l^T [Cc][R]
-    gemm(m, m->dz, m->wt[l], M, Cc, R, dz_cols, R, nullptr, m->da, nullptr, Cc, Cc, 0);
-    launch_gelu_backward(m->z[l - 1], m->da, m->dz, (int64_t)M * Cc, m->st);
-    dz_cols = Cc;
+    const int Rt = l == L - 1 ? m->out_rows : R;  // dW rows (a multiple of 128; dz^T has R of them)
+    GemmArgs g[2];
+    // dW = dz^T . a_{l-1}: A = dz^T [R][M], B = a_{l-1}^T [Cc][M]
+    g[0] = GemmArgs{m->dzt[l], m->at[l], Rt, Cc, M, M, M, nullptr, m->grad + m->w_off[l], nullptr, Cc, Cc, 0, m->d_err};
+    g[0].rows_a = R;
+    if (l > 0) {
+      // dz_{l-1} = (dz . W_l) GELU'(z_{l-1}): A = dz [M][R], B = W_l^T [Cc][R]
+      g[1] = GemmArgs{m->dz[l], m->wt[l], M, Cc, R, R, R, nullptr, nullptr, m->dz[l - 1], Cc, Cc, 0, m->d_err};
+      g[1].z = m->z[l - 1];
+      g[1].out_t = m->dzt[l - 1];
+      g[1].ldt = M;
+    }
+    gemm(m, g, l > 0 ? 2 : 1);
   }
-  MCK(cudaMemcpyAsync(m->h_part.data(), m->loss_part, mse_blocks(M) * sizeof(double), cudaMemcpyDeviceToHost, m->st));
-  MCK(cudaStreamSynchronize(m->st));
-  double s = 0.0;
-  for (int b = 0; b < mse_blocks(M); ++b) s += m->h_part[b];
-  *sse = s;
-  return FELIS_OK;
+  launch_bias_grads(layers_of(m), M, m->grad, m->st);
 }
 
 felis_status refresh_bf16(felis_mlp* m) {
@@ -226,14 +257,7 @@ felis_status adamw_step(felis_mlp* m, float lr, float wd) {
   const float b1 = 0.9f, b2 = 0.999f, eps = 1e-8f;
   m->steps += 1;
   const float bc1 = 1.f - powf(b1, (float)m->steps), bc2 = 1.f - powf(b2, (float)m->steps);
-  for (int l = 0; l < kLayers; ++l) {
-    const int64_t nw = (int64_t)m->rows[l] * m->cols[l];
-    launch_adamw(m->p + m->w_off[l], m->grad + m->w_off[l], m->m + m->w_off[l], m->v + m->w_off[l], m->wb[l], nw,
-                 lr, b1, b2, eps, wd, bc1, bc2, m->st);
-    launch_adamw(m->p + m->b_off[l], m->grad + m->b_off[l], m->m + m->b_off[l], m->v + m->b_off[l], nullptr,
-                 m->rows[l], lr, b1, b2, eps, 0.f, bc1, bc2, m->st);
-    if (l > 0) launch_transpose_bf16(m->wb[l], m->rows[l], m->cols[l], m->cols[l], m->wt[l], m->rows[l], m->cols[l], m->st);
-  }
+  launch_adamw(layers_of(m), m->p, m->grad, m->m, m->v, lr, b1, b2, eps, wd, bc1, bc2, m->st);
   MCK(cudaGetLastError());
   return FELIS_OK;
 }
@@ -327,11 +351,11 @@ felis_status felis_mlp_create(int32_t n_in, int32_t width, int32_t n_out, uint64
 void felis_mlp_destroy(felis_mlp* m) {
   if (!m) return;
   if (m->st) cudaStreamSynchronize(m->st);
-  void* ptrs[] = {m->d_err, m->p, m->grad, m->m, m->v, m->xb, m->xf, m->tgt, m->dz, m->dzt, m->at, m->da,
-                  m->loss_part, m->dx, m->dt, m->d_idx};
+  void* ptrs[] = {m->d_err, m->p, m->grad, m->m, m->v, m->xb, m->xf, m->z[kLayers - 1],
+                  m->layer_buf, m->train_buf, m->loss_part, m->dx, m->dt, m->d_idx};
   for (void* q : ptrs) if (q) cudaFree(q);
   for (int l = 0; l < kLayers; ++l) {
-    void* q[] = {m->wb[l], m->wt[l], m->z[l], m->a[l]};
+    void* q[] = {m->wb[l], m->wt[l]};
     for (void* x : q) if (x) cudaFree(x);
   }
   if (m->ev0) cudaEventDestroy(m->ev0);
@@ -382,7 +406,7 @@ felis_status felis_mlp_set_params(felis_mlp* m, const float* in) {
 felis_status felis_mlp_forward(felis_mlp* m, const float* x, int64_t n, float* y) {
   if (!m || n < 0 || (n > 0 && (!x || !y))) return mfail(m, FELIS_BAD_ARG, "bad argument");
   felis_status s =
-      ensure_cap(m, (int)std::min<int64_t>(round_up((int)std::min<int64_t>(n, kFwdChunk), 128), kFwdChunk));
+      ensure_cap(m, (int)std::min<int64_t>(round_up((int)std::min<int64_t>(n, kFwdChunk), 128), kFwdChunk), !m->fused);
   if (s != FELIS_OK) return s;
   for (int64_t r0 = 0; r0 < n; r0 += kFwdChunk) {
     const int nr = (int)std::min<int64_t>(kFwdChunk, n - r0);
@@ -422,17 +446,28 @@ felis_status felis_mlp_set_fused(felis_mlp* m, int32_t enable) {
 felis_status felis_mlp_gradients(felis_mlp* m, const float* x, const float* t, int64_t n, float* grads,
                                  double* loss) {
   if (!m || !x || !t || n < 1 || n > kChunk) return mfail(m, FELIS_BAD_ARG, "bad argument (1 <= n <= 65536)");
-  const int M = round_up((int)n, 128);
-  felis_status s = ensure_cap(m, M);
+  const int M = round_up((int)n, 128), parts = mse_blocks(M);
+  felis_status s = ensure_train(m, M, parts);
   if (s != FELIS_OK) return s;
-  MCK(cudaMemsetAsync(m->xf, 0, (size_t)M * m->in_p * sizeof(float), m->st));
-  if ((s = upload_rows(m, x, n, m->n_in, m->in_p, m->xf)) != FELIS_OK) return s;
-  launch_f32_to_bf16(m->xf, m->xb, (int64_t)M * m->in_p, m->st);
-  MCK(cudaMemsetAsync(m->tgt, 0, (size_t)M * m->out_p * sizeof(float), m->st));
-  if ((s = upload_rows(m, t, n, m->n_out, m->out_p, m->tgt)) != FELIS_OK) return s;
+  // rows and targets as they are, padded on the device by way of the first
+  // and the last layer's z, which the forward pass has not written yet (a row
+  // of z is at least 128 floats or the padded outputs; of inputs at most 256
+  // 16-bit values)
+  bf16* rows = reinterpret_cast<bf16*>(m->z[0]);
+  const CopyPart in{x, m->xf, (size_t)n * m->n_in * sizeof(float)};
+  MCK(m->stage.upload(&in, 1, m->device, m->st));
+  launch_pack_rows(m->xf, (int)n, m->n_in, M, m->in_p, rows, m->st);
+  const CopyPart tg{t, m->xf, (size_t)n * m->n_out * sizeof(float)};
+  MCK(m->stage.upload(&tg, 1, m->device, m->st));
+  launch_pad_rows(m->xf, (int)n, m->n_out, m->out_p, m->z[kLayers - 1], m->st);
+  launch_batch_rows(rows, m->z[kLayers - 1], nullptr, (int)n, M, m->in_p, m->out_p, m->xb, m->at[0], m->tgt, m->st);
   forward(m, M);
+  backward(m, M, (int)n, m->loss_part);
+  std::vector<double> part(parts);
+  MCK(cudaMemcpyAsync(part.data(), m->loss_part, parts * sizeof(double), cudaMemcpyDeviceToHost, m->st));
+  MCK(cudaStreamSynchronize(m->st));
   double sse = 0.0;
-  if ((s = backward(m, M, (int)n, &sse)) != FELIS_OK) return s;
+  for (double v : part) sse += v;
   if ((s = check_err(m)) != FELIS_OK) return s;
   std::vector<float> h(m->n_param);
   MCK(cudaMemcpy(h.data(), m->grad, h.size() * sizeof(float), cudaMemcpyDeviceToHost));
@@ -472,28 +507,36 @@ felis_status felis_mlp_train(felis_mlp* m, int32_t epochs, int32_t batch, float 
                              uint64_t seed, double* loss_per_epoch) {
   if (!m || epochs < 1 || batch < 128 || batch % 128 || batch > kChunk || m->n_data < 1)
     return mfail(m, FELIS_BAD_ARG, "bad argument (batch a multiple of 128, data set first)");
-  felis_status s = ensure_cap(m, batch);
+  const int64_t batches = (m->n_data + batch - 1) / batch;
+  const int parts = mse_blocks(batch);
+  felis_status s = ensure_train(m, batch, batches * parts);
   if (s != FELIS_OK) return s;
   std::mt19937_64 rng(seed ? seed : 1);
   std::vector<int> perm(m->n_data);
+  std::vector<double> part((size_t)(batches * parts));
   for (int64_t i = 0; i < m->n_data; ++i) perm[i] = (int)i;
   for (int ep = 0; ep < epochs; ++ep) {
     std::shuffle(perm.begin(), perm.end(), rng);
     MCK(cudaMemcpyAsync(m->d_idx, perm.data(), perm.size() * sizeof(int), cudaMemcpyHostToDevice, m->st));
-    double sse = 0.0;
-    for (int64_t b0 = 0; b0 < m->n_data; b0 += batch) {
+    // the batches of an epoch follow one another on the stream; their losses
+    // are read once at its end
+    for (int64_t b = 0; b < batches; ++b) {
+      const int64_t b0 = b * batch;
       const int nr = (int)std::min<int64_t>(batch, m->n_data - b0);
       const int M = round_up(nr, 128);
-      k_gather_rows<<<nr, 64, 0, m->st>>>(m->dx, m->dt, m->d_idx + b0, nr, m->in_p, m->out_p, m->xb, m->tgt);
-      if (M > nr) {
-        k_zero_rows_bf16<<<64, 256, 0, m->st>>>(m->xb, (int64_t)nr * m->in_p, (int64_t)M * m->in_p);
-        MCK(cudaMemsetAsync(m->tgt + (size_t)nr * m->out_p, 0, (size_t)(M - nr) * m->out_p * sizeof(float), m->st));
-      }
+      launch_batch_rows(m->dx, m->dt, m->d_idx + b0, nr, M, m->in_p, m->out_p, m->xb, m->at[0], m->tgt, m->st);
       forward(m, M);
-      double part = 0.0;
-      if ((s = backward(m, M, nr, &part)) != FELIS_OK) return s;
-      sse += part;
+      backward(m, M, nr, m->loss_part + b * parts);
       if ((s = adamw_step(m, lr, weight_decay)) != FELIS_OK) return s;
+    }
+    MCK(cudaMemcpyAsync(part.data(), m->loss_part, part.size() * sizeof(double), cudaMemcpyDeviceToHost, m->st));
+    MCK(cudaStreamSynchronize(m->st));
+    double sse = 0.0;
+    for (int64_t b = 0; b < batches; ++b) {
+      const int nr = (int)std::min<int64_t>(batch, m->n_data - b * batch), np = mse_blocks(round_up(nr, 128));
+      double sum = 0.0;
+      for (int k = 0; k < np; ++k) sum += part[(size_t)(b * parts + k)];
+      sse += sum;
     }
     if (loss_per_epoch) loss_per_epoch[ep] = sse / ((double)m->n_data * m->n_out);
   }

@@ -108,5 +108,13 @@ __device__ __forceinline__ float gelu_f(float z) {
   return 0.5f * z * (1.f + tanh_hw(u));
 }
 
+// Its derivative: with t = tanh(u), u = c (z + a z^3):
+// 0.5 (1 + t) + 0.5 z (1 - t^2) c (1 + 3 a z^2).
+__device__ __forceinline__ float gelu_grad(float z) {
+  const float c = 0.79788456080286536f, a = 0.044715f;
+  const float t = tanh_hw(c * fmaf(a * z, z * z, z));
+  return 0.5f * (1.f + t) + 0.5f * z * (1.f - t * t) * c * fmaf(3.f * a * z, z, 1.f);
+}
+
 }  // namespace tc
 }  // namespace felis

@@ -49,6 +49,15 @@ cudaError_t HostStage::run(const CopyPart* parts, int nparts, Mode mode, int dev
       total += n;
     }
   if (!total) return cudaSuccess;
+  if (!pinned_ && total < kChunk && mode != kDownWiden) {
+    // too little to page-lock memory for (2 ms)
+    for (const CopyPart& c : chunks) {
+      const cudaError_t x = mode == kUp ? cudaMemcpyAsync(c.dst, c.src, c.bytes, cudaMemcpyHostToDevice, st)
+                                        : cudaMemcpyAsync(c.dst, c.src, c.bytes, cudaMemcpyDeviceToHost, st);
+      if (x != cudaSuccess) return x;
+    }
+    return cudaStreamSynchronize(st);
+  }
   // one thread per 4 MB, as far as the machine has cores
   const int cores = std::max(1, (int)std::thread::hardware_concurrency());
   const int threads = (int)std::min<size_t>(std::min(kThreads, cores), (total >> 22) + 1);
@@ -58,7 +67,7 @@ cudaError_t HostStage::run(const CopyPart* parts, int nparts, Mode mode, int dev
   std::atomic<int> status{cudaSuccess};
   auto work = [&](int t) {
     char* slot = pinned_ + (size_t)t * kSlots * kChunk;
-    size_t held[kSlots];
+    size_t held[kSlots] = {};
     bool busy[kSlots] = {};  // a copy through the slot is in flight
     auto fail = [&](cudaError_t x) {
       int ok = cudaSuccess;
