@@ -85,6 +85,8 @@ struct felis_handle {
   int4* box = nullptr;
   double2* Ez = nullptr;
   int ring_base = 0;
+  int* lit = nullptr;    // per plane: 0 if it is known to be zero everywhere (written by the ADI)
+  bool handed_out = false;  // the caller holds plane addresses and may write there unseen
   // tables
   double* d_bessel = nullptr;
   std::vector<double> bessel_host;
@@ -500,7 +502,14 @@ felis_status run_adi(felis_handle* h, int use_source) {
   a.ring_base = h->ring_base;
   a.Sc = h->Sc;
   a.box = h->box;
-  a.use_source = use_source;
+  double Phi;
+  cd etaX, etaY;
+  // the deposit's sources (of the same h->lat, solve_field_impl) are multiples of eta
+  const bool known = polarisation(h->lat, &Phi, &etaX, &etaY);
+  a.use_source[0] = use_source && (!known || etaX.re != 0.0 || etaX.im != 0.0);
+  a.use_source[1] = use_source && (!known || etaY.re != 0.0 || etaY.im != 0.0);
+  a.lit = h->lit;
+  a.skip = !h->handed_out;
   a.tab = h->d_adi;
   a.energy = h->d_planes;
   a.nxp = h->nxp;
@@ -703,6 +712,8 @@ felis_status felis_create(const felis_params* p, felis_handle** out) {
   const size_t N = (size_t)nx * ny;
   if (ce == cudaSuccess) ce = cudaMalloc(&h->U, (size_t)H * 2 * S * N * sizeof(double2));
   if (ce == cudaSuccess) ce = cudaMemsetAsync(h->U, 0, (size_t)H * 2 * S * N * sizeof(double2), h->st);
+  if (ce == cudaSuccess) ce = cudaMalloc(&h->lit, (size_t)H * 2 * S * sizeof(int));
+  if (ce == cudaSuccess) ce = cudaMemsetAsync(h->lit, 0, (size_t)H * 2 * S * sizeof(int), h->st);
   if (ce == cudaSuccess) ce = cudaMalloc(&h->Sc, (size_t)H * 2 * S * N * sizeof(double2));
   if (ce == cudaSuccess) ce = cudaMalloc(&h->box, (size_t)S * sizeof(int4));
   const size_t ezn = (size_t)p->scl_mode * (S + 2) * p->scf_mode * p->nr;
@@ -814,7 +825,7 @@ felis_status felis_create(const felis_params* p, felis_handle** out) {
 void felis_destroy(felis_handle* h) {
   if (!h) return;
   if (h->st) cudaStreamSynchronize(h->st);
-  void* ptrs[] = {h->x, h->y, h->px, h->py, h->th, h->ga, h->d_soff, h->d_weight, h->d_tiles, h->U, h->Sc, h->box,
+  void* ptrs[] = {h->x, h->y, h->px, h->py, h->th, h->ga, h->d_soff, h->d_weight, h->d_tiles, h->U, h->lit, h->Sc, h->box,
                   h->Ez, h->d_bessel, h->d_wake, h->d_log, h->d_radial, h->d_adi, h->d_part, h->d_planes, h->d_planes2,
                   h->d_hist_e, h->d_hist_t, h->d_hist_b, h->d_tmp, h->d_l1, h->d_err,
                   h->dep.key, h->dep.rkey, h->dep.wx1, h->dep.wy1, h->dep.wr1, h->dep.coef, h->dep.fx, h->dep.fy, h->dep.ez,
@@ -907,6 +918,7 @@ felis_status felis_upload_field(felis_handle* h, int32_t hidx, int32_t pol, cons
   // the ring holds the slices in two runs of planes
   const int run = S - h->ring_base;  // slices 0 .. run - 1 sit at ring_base ..
   double2* P = h->U + (size_t)(hidx * 2 + pol) * S * N;
+  CK(cudaMemsetAsync(h->lit + (size_t)(hidx * 2 + pol) * S, 1, S * sizeof(int), h->st));  // until the ADI has seen them
   CK(cudaMemcpyAsync(P + (size_t)h->ring_base * N, data + 2 * N, (size_t)run * N * sizeof(double2),
                      cudaMemcpyHostToDevice, h->st));
   if (run < S)
@@ -1423,6 +1435,7 @@ felis_status felis_first_planes_device(felis_handle* h, double** planes) {
   for (int hh = 0; hh < H; ++hh)
     for (int pol = 0; pol < 2; ++pol)
       planes[hh * 2 + pol] = reinterpret_cast<double*>(h->U + field_plane(S, hh, pol, 0, h->ring_base) * N);
+  h->handed_out = true;
   h->diag_valid = false;
   return FELIS_OK;
 }
@@ -1444,6 +1457,8 @@ felis_status felis_set_first_planes(felis_handle* h, const double* in) {
     for (int pol = 0; pol < 2; ++pol)
       CK(cudaMemcpy(h->U + field_plane(S, hh, pol, 0, h->ring_base) * N, in + 2 * ((size_t)(hh * 2 + pol) * N),
                     N * sizeof(double2), cudaMemcpyHostToDevice));
+  for (int k = 0; k < 2 * H; ++k)
+    CK(cudaMemsetAsync(h->lit + field_plane(S, k >> 1, k & 1, 0, h->ring_base), 1, sizeof(int), h->st));
   h->diag_valid = false;
   return FELIS_OK;
 }

@@ -56,6 +56,7 @@ struct Inst {
   int64_t* soff = nullptr;
   float* weight = nullptr;
   float2* U = nullptr;
+  int* lit = nullptr;
   float2* Ez = nullptr;
   float* d_bessel = nullptr;
   double* wake = nullptr;
@@ -406,7 +407,7 @@ felis_status upload_inst_table(felis_batch* b) {
     D.ks = p.ks; D.dz = p.dz; D.dx = p.dx; D.dy = p.dy; D.dr = p.dr; D.minX = p.min_x; D.minY = p.min_y;
     D.gamR = p.gam_r; D.dBessel = p.d_bessel;
     D.x = I.x; D.y = I.y; D.px = I.px; D.py = I.py; D.dg = I.dg; D.th = I.th;
-    D.soff = I.soff; D.weight = I.weight; D.U = I.U; D.Ez = I.Ez; D.src = I.src; D.sbox = I.sbox;
+    D.soff = I.soff; D.weight = I.weight; D.U = I.U; D.lit = I.lit; D.Ez = I.Ez; D.src = I.src; D.sbox = I.sbox;
     D.bessel = I.d_bessel; D.wakeE = I.wake;
     D.adi_c = I.adi; D.part_e = I.part_e; D.part_b = I.part_b; D.err = I.err;
   }
@@ -793,6 +794,8 @@ felis_status felis_batch_create(const felis_params* const* instances, int32_t n,
     const size_t un = (size_t)H * 2 * S * N;
     if (e == cudaSuccess) e = cudaMalloc(&I.U, un * sizeof(float2));
     if (e == cudaSuccess) e = cudaMemset(I.U, 0, un * sizeof(float2));
+    if (e == cudaSuccess) e = cudaMalloc(&I.lit, (size_t)H * 2 * S * sizeof(int));
+    if (e == cudaSuccess) e = cudaMemset(I.lit, 0, (size_t)H * 2 * S * sizeof(int));
     const size_t ezn = (size_t)p->scl_mode * S * p->scf_mode * p->nr;
     if (e == cudaSuccess) e = cudaMalloc(&I.Ez, ezn * sizeof(float2));
     if (e == cudaSuccess) e = cudaMemset(I.Ez, 0, ezn * sizeof(float2));
@@ -842,7 +845,7 @@ void felis_batch_destroy(felis_batch* b) {
   if (!b) return;
   if (b->st) cudaStreamSynchronize(b->st);
   for (auto& I : b->in) {
-    void* ptrs[] = {I.x, I.y, I.px, I.py, I.dg, I.th, I.soff, I.weight, I.U, I.Ez, I.d_bessel, I.wake, I.adi,
+    void* ptrs[] = {I.x, I.y, I.px, I.py, I.dg, I.th, I.soff, I.weight, I.U, I.lit, I.Ez, I.d_bessel, I.wake, I.adi,
                     I.src, I.sbox, I.part_e, I.part_b, I.err};
     for (void* q : ptrs) if (q) cudaFree(q);
   }
@@ -952,6 +955,7 @@ felis_status felis_batch_upload_field(felis_batch* b, int32_t inst, int32_t hidx
   BCK(ensure_stage(b, std::max(plane_bytes, std::min((size_t)S * plane_bytes, (size_t)64 << 20))));
   const int per = (int)std::max<size_t>(1, b->stage_bytes / plane_bytes);
   float2* U = I.U + (size_t)(hidx * 2 + pol) * S * N;
+  BCK(cudaMemsetAsync(I.lit + (size_t)(hidx * 2 + pol) * S, 1, S * sizeof(int), b->st));  // until the ADI has seen them
   for (int s0 = 0; s0 < S; s0 += per) {
     const int ns = std::min(per, S - s0);
     BCK(cudaMemcpyAsync(b->stage, data + 2 * (size_t)(s0 + 1) * N, (size_t)ns * plane_bytes, cudaMemcpyDefault, b->st));

@@ -35,6 +35,7 @@ struct BInst {
   const int64_t* soff;   // [S+1]
   const float* weight;   // [S]
   float2* U;             // [H][2][S][N] ring per (H, pol)
+  int* lit;              // [H][2][S] ring: 0 if the plane is known to be zero everywhere
   float2* Ez;            // [L][S][F][nr]
   float2* src;           // [S][nsrc][N] source of the next ADI, box-compact
   int4* sbox;            // [S] cell box of that source (bi0, bi1, bj0, bj1)

@@ -28,7 +28,9 @@ struct AdiLaunch {
   int ring_base;
   const double2* Sc;   // [H][2][S][N]
   const int4* box;     // per slice: {i0, i1, j0, j1} of written source cells
-  int use_source;      // currentFlag of solveField
+  int use_source[2];   // currentFlag of solveField and a source in this polarisation
+  int* lit;            // [H][2][S] ring: 0 if the plane is known to be zero everywhere
+  int skip;            // planes may be skipped by it
   const AdiTab* tab;   // [H] (device array of structs)
   double* energy;      // [H][2][S] plane sums of |U|^2 after the solve (may be null)
   int nxp;             // padded row length of the shared-memory plane

@@ -260,7 +260,18 @@ __global__ void __launch_bounds__(1024) k_batch_adi(BatchLaunch a) {
   // to whole warps get no line (l = NL fails every line test below)
   int q = tid / NL, l = tid - q * NL;
   if (q > 3) { q = 3; l = NL; }
-  float2* U = I.U + ((size_t)hp * S + (s + T.ring_base) % S) * I.N;
+  const int phys = (s + T.ring_base) % S;
+  float2* U = I.U + ((size_t)hp * S + phys) * I.N;
+  // A plane that holds nothing and receives nothing stays as it is: the sweeps
+  // of zeros give zeros.  A planar undulator drives one polarisation, so half
+  // of its planes are of this kind (1024 slices of 102 x 102: 0.213 -> 0.123 ms).
+  const float2 sfac = T.sfac[h][pol];
+  const bool driven = T.current && (sfac.x != 0.f || sfac.y != 0.f);
+  int* lit = I.lit + (size_t)hp * S + phys;
+  if (!driven && *lit == 0) {
+    if (tid == 0) I.part_e[(size_t)s * 2 * I.H + hp] = 0.0;
+    return;
+  }
   const float2* ad = I.adi_c + (size_t)h * 16 * Mx;
   float2* pl = reinterpret_cast<float2*>(sm);  // interior cells, [my][P]
   float2* tb = pl + (size_t)my * P;            // 16 tables of Mx
@@ -289,8 +300,7 @@ __global__ void __launch_bounds__(1024) k_batch_adi(BatchLaunch a) {
   // polarisations), even harmonic its own plane
   int bi0 = 1, bi1 = 0, bj0 = 1, bj1 = 0, bw = 0;
   const float2* Sc = nullptr;
-  const float2 sfac = T.sfac[h][pol];
-  if (T.current) {
+  if (driven) {
     const int4 b = I.sbox[s];
     bi0 = b.x; bi1 = b.y; bj0 = b.z; bj1 = b.w;
     bw = bi1 - bi0 + 1;
@@ -322,6 +332,7 @@ __global__ void __launch_bounds__(1024) k_batch_adi(BatchLaunch a) {
   const int c0 = I.cx[q], c1 = I.cx[q + 1];  // this thread's chunk of a row (x sweep)
   const int r0 = I.cy[q], r1 = I.cy[q + 1];  // and of a column (x right-hand side, y sweep)
   double e = 0.0;
+  int any = 0;  // bits of every value of the plane after the solve
   // ---- x sweep right-hand side: thread (column l, row chunk q), in place in
   // the staged plane; the rows either side of the chunk are read first
   {
@@ -340,6 +351,7 @@ __global__ void __launch_bounds__(1024) k_batch_adi(BatchLaunch a) {
       else if (k < 2 * nx) v = U[(size_t)(ny - 1) * nx + (k - nx)];
       else v = U[(size_t)(((k - 2 * nx) >> 1) + 1) * nx + (((k - 2 * nx) & 1) ? nx - 1 : 0)];
       e += (double)(v.x * v.x + v.y * v.y);
+      any |= __float_as_int(v.x) | __float_as_int(v.y);
     }
     __syncthreads();
     if (valid) {
@@ -472,6 +484,7 @@ __global__ void __launch_bounds__(1024) k_batch_adi(BatchLaunch a) {
         const float2 xn = v[(r + 1) * P];
         Ug[(size_t)r * nx] = x;
         e += (double)(x.x * x.x + x.y * x.y);
+        any |= __float_as_int(x.x) | __float_as_int(x.y);
         x = xn;
       }
       for (int r = rq; r < r1; ++r) {
@@ -479,12 +492,17 @@ __global__ void __launch_bounds__(1024) k_batch_adi(BatchLaunch a) {
         const float2 o = cad(x, cm(pQ[r], uin));
         Ug[(size_t)r * nx] = o;
         e += (double)(o.x * o.x + o.y * o.y);
+        any |= __float_as_int(o.x) | __float_as_int(o.y);
         x = xn;
       }
     }
   }
   const double et = block_sum_d(e, redd);
-  if (tid == 0) I.part_e[(size_t)s * 2 * I.H + hp] = et;
+  any = __syncthreads_or(any & 0x7fffffff);
+  if (tid == 0) {
+    I.part_e[(size_t)s * 2 * I.H + hp] = et;
+    *lit = any;
+  }
 }
 
 // ============================================================================
