@@ -84,7 +84,10 @@ struct BStep {
   int64_t rad_off;
 };
 
-constexpr int kPushThreads = 128;  // threads per CTA of the push launch
+// Threads per CTA of the push launch: a multiple of 128, at most what one CTA of
+// the instance may have at its register budget.
+constexpr int kPushThreads = 128;
+int batch_push_threads_max(int H);
 
 struct BatchLaunch {
   const BInst* inst;
@@ -93,6 +96,7 @@ struct BatchLaunch {
   int nwork;
   int smem_bytes;     // dynamic shared memory of the launch
   int mode;           // push launch: BATCH_PUSH or BATCH_DEPOSIT_ONLY
+  int threads;        // push launch: threads per CTA, a multiple of 128
   const double* rad;  // push launch: the radial elimination tables of the run (BStep::rad_off)
 };
 
@@ -109,8 +113,8 @@ cudaError_t launch_f32_to_f64(const float* src, double* dst, int64_t n, double o
 cudaError_t launch_field_to_f32(const double* src, float2* U, int s0, int ns, int S, int N, int ring_base,
                                 cudaStream_t st);
 // H: the largest harmonic count of the ensemble (selects the kernel instance).
-// The push launch: 128 threads per CTA (kPushThreads), the instance of the
-// ensemble's largest harmonic count H and Ez mode count L.
+// The push launch: the instance of the ensemble's largest harmonic count H and
+// Ez mode count L.
 void launch_batch_push(const BatchLaunch& a, int H, int L, cudaStream_t st);
 void launch_batch_measure(const BInst* inst, const BStep* step, const int4* work, int nwork, cudaStream_t st);
 // Per instance {sum |U|^2, Re, Im sum conj(U_s) U_{s+1}} of harmonic index

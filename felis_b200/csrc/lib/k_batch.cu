@@ -654,7 +654,8 @@ __device__ __forceinline__ void deposit_pass(const float* __restrict__ xs, const
                                              int ny, int bi0, int bi1, int bj0, int bj1, int bw, int cells,
                                              int wi0, int wi1, int wj0, int wj1, int wcells, float iq2, float iqr,
                                              acc_t* gacc, unsigned sacc, unsigned sR, float dr, float idr2, int nr,
-                                             int L, int F, float (&acc7)[7], float (&bre)[HM], float (&bim)[HM]) {
+                                             int L, int F, float (&acc7)[7], float (&bre)[HM], float (&bim)[HM],
+                                             int apart) {
   const int ww = wi1 - wi0 + 1;
   float2 ePhi[HM];  // e^{-i H Phi/2} of the deposit's lattice
 #pragma unroll
@@ -663,7 +664,7 @@ __device__ __forceinline__ void deposit_pass(const float* __restrict__ xs, const
   // first reads find the push's latest stores still in L2.  The next
   // particle's state is loaded one iteration ahead: the accumulator adds below
   // are compiler memory barriers, so no load moves above them.
-  const int nt = blockDim.x, t0 = threadIdx.x;
+  const int nt = blockDim.x - apart, t0 = threadIdx.x - apart;  // the first threads of a wide CTA take the sums
   float nxv = 0.f, nyv = 0.f, ndg = 0.f, npx = 0.f, npy = 0.f;
   double nth = 0.0;
   const int qlast = t0 < P ? t0 + (P - 1 - t0) / nt * nt : -1;  // this thread's last particle
@@ -791,9 +792,20 @@ template <int HM>
 struct PushBlocks {
   static constexpr int value = HM == 1 ? 7 : (HM == 2 ? 5 : 4);
 };
+// The instances for few slices (WIDE) have the threads of all those CTAs, less
+// what one CTA may have, in one.  A thread's particles are independent and the
+// deposit adds integers; the beam's sums are taken by 128 threads in the order
+// of a CTA of 128, so that both give the same bits.  One slice of 8192 particles:
+// 0.155 ms with 128 threads, 0.065 with 896.
+template <int HM>
+struct PushWide {
+  static constexpr int value = HM == 1 ? 896 : (HM == 2 ? 640 : 512);
+};
 
-template <int HM, int LM>
-__global__ void __launch_bounds__(kPushThreads, PushBlocks<HM>::value) k_batch_push(BatchLaunch a) {
+template <int HM, int LM, bool WIDE>
+__global__ void __launch_bounds__(WIDE ? PushWide<HM>::value : kPushThreads, WIDE ? 1 : PushBlocks<HM>::value)
+    k_batch_push(BatchLaunch a) {
+  constexpr int kWarps = (WIDE ? PushWide<HM>::value : kPushThreads) / 32;
   extern __shared__ __align__(16) unsigned char sm[];
   __shared__ __align__(16) float smap[48];  // transverse map: D0, M1, M2 (row-major 4x4 each)
   __shared__ __align__(8) unsigned long long fbar;  // bulk staging of the field box
@@ -1175,11 +1187,14 @@ __global__ void __launch_bounds__(kPushThreads, PushBlocks<HM>::value) k_batch_p
   for (int h = 0; h < HM; ++h) { bre[h] = 0.f; bim[h] = 0.f; }
   // the 7 + 2 H + 1 block sums of the beam, each as block_sum_d forms it (warp
   // tree, then the warps in order), under one barrier
+  // the threads that hold them (a constant here unrolls the loops below and
+  // with their code the two-harmonic launch took 0.44 ms instead of 0.395)
+  const int snt = WIDE ? kPushThreads : nt;
   __shared__ double rsum[kPushThreads / 32][7 + 2 * HM + 1];
   auto write_sums = [&]() {
     const int stride = 7 + 2 * H + 1;
     double* out = I.part_b + (size_t)s * stride;
-    const double wsum = (double)weight * (double)max(0, (P - tid + nt - 1) / nt);
+    const double wsum = (double)weight * (double)max(0, (P - tid + snt - 1) / snt);
     double v[7 + 2 * HM + 1];
 #pragma unroll
     for (int k = 0; k < 7; ++k) v[k] = (double)acc7[k];
@@ -1189,6 +1204,7 @@ __global__ void __launch_bounds__(kPushThreads, PushBlocks<HM>::value) k_batch_p
     const int w = tid >> 5, ln = tid & 31;
 #pragma unroll
     for (int k = 0; k < 7 + 2 * HM + 1; ++k) {
+      if (WIDE && w >= kPushThreads / 32) break;
       if (k >= 7 + 2 * H && k < 7 + 2 * HM) continue;  // harmonics beyond H
       double x = v[k];
       for (int o = 16; o > 0; o >>= 1) x += __shfl_down_sync(0xffffffffu, x, o);
@@ -1198,7 +1214,7 @@ __global__ void __launch_bounds__(kPushThreads, PushBlocks<HM>::value) k_batch_p
     if (tid == 0) {
       auto total = [&](int k) {
         double t = 0.0;
-        for (int q = 0; q < (nt + 31) / 32; ++q) t += rsum[q][k];
+        for (int q = 0; q < (snt + 31) / 32; ++q) t += rsum[q][k];
         return t;
       };
       for (int k = 0; k < 7; ++k) out[k] = total(k);
@@ -1207,12 +1223,13 @@ __global__ void __launch_bounds__(kPushThreads, PushBlocks<HM>::value) k_batch_p
     }
   };
   if (push && !dep) {
-    for (int q = tid; q < P; q += nt) {
-      const int64_t n = p0 + q;
-      float2 eb[HM];
-      harmonic_phases<HM>(eb, hh, H, theta_red(ths[n]));
-      beam_sums<HM>(acc7, bre, bim, eb, H, xs[n], ys[n], pxs[n], pys[n], gRf + dgs[n]);
-    }
+    if (!WIDE || tid < kPushThreads)
+      for (int q = tid; q < P; q += snt) {
+        const int64_t n = p0 + q;
+        float2 eb[HM];
+        harmonic_phases<HM>(eb, hh, H, theta_red(ths[n]));
+        beam_sums<HM>(acc7, bre, bim, eb, H, xs[n], ys[n], pxs[n], pys[n], gRf + dgs[n]);
+      }
     write_sums();
   }
   if (!dep) return;
@@ -1220,35 +1237,36 @@ __global__ void __launch_bounds__(kPushThreads, PushBlocks<HM>::value) k_batch_p
   // bounds: |w mc| <= wm H weight coef_U / g for odd harmonics, times |f| <=
   // 2 xi2 H for even ones (|eta| <= 1, |e| = 1); radial |w c| <= coef_Ez L
   // weight (1 + |wr1|) / max(ir, 1)
-  const float bmax = wfmax > 0.f ? wfmax / gmin : 0.f, rmax = rin ? 1.625f : 0.f;
+  const float rmax = rin ? 1.625f : 0.f;
   // the cell box and both bounds over the CTA: warp trees, then the warps,
   // one barrier for the six values
   int mi0, mi1, mj0, mj1;
   float bmx, rmx;
   {
-    __shared__ int rbox[kPushThreads / 32][4];
-    __shared__ float rbnd2[kPushThreads / 32][2];
+    __shared__ int rbox[kWarps][4];
+    __shared__ float rbnd2[kWarps][3];
     int iv[4] = {ci0, -ci1, cj0, -cj1};
-    float fv[2] = {bmax, rmax};
+    float fv[3] = {wfmax, rmax, -gmin};  // extremes of the slice, the same in every launch shape
 #pragma unroll
     for (int k = 0; k < 4; ++k)
       for (int o = 16; o > 0; o >>= 1) iv[k] = min(iv[k], __shfl_down_sync(0xffffffffu, iv[k], o));
 #pragma unroll
-    for (int k = 0; k < 2; ++k)
+    for (int k = 0; k < 3; ++k)
       for (int o = 16; o > 0; o >>= 1) fv[k] = fmaxf(fv[k], __shfl_down_sync(0xffffffffu, fv[k], o));
     if ((tid & 31) == 0) {
       for (int k = 0; k < 4; ++k) rbox[tid >> 5][k] = iv[k];
-      for (int k = 0; k < 2; ++k) rbnd2[tid >> 5][k] = fv[k];
+      for (int k = 0; k < 3; ++k) rbnd2[tid >> 5][k] = fv[k];
     }
     __syncthreads();
     int t[4] = {1 << 30, 1 << 30, 1 << 30, 1 << 30};
-    float u[2] = {0.f, 0.f};
+    float u[3] = {0.f, 0.f, -3.0e38f};
     for (int q = 0; q < (nt + 31) / 32; ++q) {
       for (int k = 0; k < 4; ++k) t[k] = min(t[k], rbox[q][k]);
-      for (int k = 0; k < 2; ++k) u[k] = fmaxf(u[k], rbnd2[q][k]);
+      for (int k = 0; k < 3; ++k) u[k] = fmaxf(u[k], rbnd2[q][k]);
     }
     mi0 = t[0]; mi1 = -t[1]; mj0 = t[2]; mj1 = -t[3];
-    bmx = u[0]; rmx = u[1];
+    bmx = u[0] > 0.f ? u[0] / -u[2] : 0.f;
+    rmx = u[1];
   }
   const float tb = bmx * 1.0625f * Hmax * weight * fabsf(D.coef_U), bnd = tb * (float)P;
   const float rtb = rmx * 1.0625f * L * weight * fabsf(D.coef_Ez), rbnd = rtb * (float)P;
@@ -1279,16 +1297,38 @@ __global__ void __launch_bounds__(kPushThreads, PushBlocks<HM>::value) k_batch_p
   const unsigned sRa = (unsigned)__cvta_generic_to_shared(sR);
   auto dep_pass = [&](auto sh_c, auto sums_c) {
     constexpr bool SHc = decltype(sh_c)::value, SUMSc = decltype(sums_c)::value;
+    const int apart = WIDE && push ? kPushThreads : 0;
     if constexpr (SHc)
       deposit_pass<HM, SHc, SUMSc>(xs, ys, pxs, pys, dgs, ths, p0, P, hh, sp, H, has_even, D, B, weight, gRf, minX,
                                    minY, idx_, idy_, nx, ny, bi0, bi1, bj0, bj1, bw, cells, 1, 0, 1, 0, 0, iq2, iqr,
-                                   nullptr, sacc, sRa, dr, idr2, nr, L, F, acc7, bre, bim);
+                                   nullptr, sacc, sRa, dr, idr2, nr, L, F, acc7, bre, bim, apart);
     else
       deposit_pass<HM, SHc, SUMSc>(xs, ys, pxs, pys, dgs, ths, p0, P, hh, sp, H, has_even, D, B, weight, gRf, minX,
                                    minY, idx_, idy_, nx, ny, bi0, bi1, bj0, bj1, bw, cells, wi0, wi1, wj0, wj1, wcells,
-                                   iq2, iqr, acc, sacc, sRa, dr, idr2, nr, L, F, acc7, bre, bim);
+                                   iq2, iqr, acc, sacc, sRa, dr, idr2, nr, L, F, acc7, bre, bim, apart);
   };
-  if (in_smem) {
+  if constexpr (WIDE) {
+    // the first 128 threads take the sums while the others deposit: a thread's
+    // particles in the deposit pass's order, the next one's state loaded ahead
+    auto sums_apart = [&]() {
+      float x = 0.f, y = 0.f, px = 0.f, py = 0.f, dg = 0.f;
+      double th = 0.0;
+      auto fetch = [&](int64_t n) { x = xs[n]; y = ys[n]; px = pxs[n]; py = pys[n]; dg = dgs[n]; th = ths[n]; };
+      int q = tid < P ? tid + (P - 1 - tid) / kPushThreads * kPushThreads : -1;
+      if (q >= 0) fetch(p0 + q);
+      for (; q >= 0; q -= kPushThreads) {
+        const float cx = x, cy = y, cpx = px, cpy = py, g = gRf + dg;
+        const float thr = theta_red(th);
+        if (q >= kPushThreads) fetch(p0 + q - kPushThreads);
+        float2 eb[HM];
+        harmonic_phases<HM>(eb, hh, H, thr);
+        beam_sums<HM>(acc7, bre, bim, eb, H, cx, cy, cpx, cpy, g);
+      }
+    };
+    if (push && tid < kPushThreads) sums_apart();
+    else if (in_smem) dep_pass(std::true_type{}, std::false_type{});
+    else dep_pass(std::false_type{}, std::false_type{});
+  } else if (in_smem) {
     if (push) dep_pass(std::true_type{}, std::true_type{});
     else dep_pass(std::true_type{}, std::false_type{});
   } else {
@@ -1486,16 +1526,23 @@ __global__ void __launch_bounds__(256) k_batch_spectrum(const BInst* inst, const
 // Instances by the largest harmonic count and the largest number of
 // longitudinal Ez modes (sizes of the register arrays).
 typedef void (*PushKernel)(BatchLaunch);
-template <int LM>
+template <int LM, bool WIDE>
 PushKernel push_kernel_l(int H) {
-  if (H <= 1) return k_batch_push<1, LM>;
-  if (H <= 2) return k_batch_push<2, LM>;
-  if (H <= 4) return k_batch_push<4, LM>;
-  return k_batch_push<FELIS_MAX_HARMONY, LM>;
+  if (H <= 1) return k_batch_push<1, LM, WIDE>;
+  if (H <= 2) return k_batch_push<2, LM, WIDE>;
+  if (H <= 4) return k_batch_push<4, LM, WIDE>;
+  return k_batch_push<FELIS_MAX_HARMONY, LM, WIDE>;
 }
-PushKernel push_kernel(int H, int L) { return L <= 1 ? push_kernel_l<1>(H) : push_kernel_l<4>(H); }
+PushKernel push_kernel(int H, int L, bool wide) {
+  if (wide) return L <= 1 ? push_kernel_l<1, true>(H) : push_kernel_l<4, true>(H);
+  return L <= 1 ? push_kernel_l<1, false>(H) : push_kernel_l<4, false>(H);
+}
 
 }  // namespace
+
+int batch_push_threads_max(int H) {
+  return H <= 1 ? PushWide<1>::value : (H <= 2 ? PushWide<2>::value : PushWide<FELIS_MAX_HARMONY>::value);
+}
 
 size_t batch_adi_smem(int nx_max, int ny_max, int src_cells) {
   const int M = nx_max > ny_max ? nx_max : ny_max;
@@ -1519,7 +1566,9 @@ size_t batch_push_smem(int nsrc_max, int LF_max, int nr_max, int box_cells) {
 
 cudaError_t batch_set_smem(int H, int L, int adi_bytes, int push_bytes) {
   cudaError_t e = cudaFuncSetAttribute(k_batch_adi, cudaFuncAttributeMaxDynamicSharedMemorySize, adi_bytes);
-  if (e == cudaSuccess) e = cudaFuncSetAttribute(push_kernel(H, L), cudaFuncAttributeMaxDynamicSharedMemorySize, push_bytes);
+  for (bool wide : {false, true})
+    if (e == cudaSuccess)
+      e = cudaFuncSetAttribute(push_kernel(H, L, wide), cudaFuncAttributeMaxDynamicSharedMemorySize, push_bytes);
   return e;
 }
 
@@ -1580,7 +1629,7 @@ void launch_batch_adi(const BatchLaunch& a, int threads, cudaStream_t st) {
 }
 
 void launch_batch_push(const BatchLaunch& a, int H, int L, cudaStream_t st) {
-  if (a.nwork > 0) push_kernel(H, L)<<<a.nwork, kPushThreads, a.smem_bytes, st>>>(a);
+  if (a.nwork > 0) push_kernel(H, L, a.threads > kPushThreads)<<<a.nwork, a.threads, a.smem_bytes, st>>>(a);
 }
 
 void launch_batch_measure(const BInst* inst, const BStep* step, const int4* work, int nwork, cudaStream_t st) {
