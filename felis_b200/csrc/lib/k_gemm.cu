@@ -67,6 +67,20 @@ struct TmaPair {
   int* err;
 };
 
+// Two neighbouring columns as BF16, through GELU where the product has it.
+__device__ __forceinline__ uint32_t pack(const TmaGemm& g, int col, float x0, float x1) {
+  if (g.gelu) {
+    if (col < g.n_valid) x0 = gelu_f(x0);
+    if (col + 1 < g.n_valid) x1 = gelu_f(x1);
+  }
+  const __nv_bfloat162 p2 = __floats2bfloat162_rn(x0, x1);
+  return *reinterpret_cast<const uint32_t*>(&p2);
+}
+
+// ONE: a single product of whole rows without z and out_t (inference by the
+// layer chain, whose epilogues bound it: the four layers of a million rows
+// take 3.31 ms in the general instance, 2.27 in this one).
+template <bool ONE>
 __global__ void __launch_bounds__(kThreads, 1) k_gemm_tma(const __grid_constant__ TmaPair P) {
   extern __shared__ unsigned char smraw[];
   __shared__ __align__(8) uint64_t full[kStages], empty[kStages], tfull[2], tempty[2];
@@ -113,8 +127,8 @@ __global__ void __launch_bounds__(kThreads, 1) k_gemm_tma(const __grid_constant_
       uint32_t ph = 0;
       bool ok = true;
       for (int t = blockIdx.x; t < ntiles && ok; t += gridDim.x) {
-        const int p = t >= P.tiles0, tp = p ? t - P.tiles0 : t, m = tp / P.g[p].nt * kBM;
-        const int n0 = tp % P.g[p].nt * P.g[p].bn;
+        const int p = !ONE && t >= P.tiles0, tp = p ? t - P.tiles0 : t, m = (ONE ? tp : tp / P.g[p].nt) * kBM;
+        const int n0 = ONE ? 0 : tp % P.g[p].nt * P.g[p].bn;
         const int nk = (P.g[p].K + kBK - 1) / kBK;
         const uint32_t bytes = kABytes + (uint32_t)P.g[p].bn * kBK * 2;
         for (int k = 0; k < nk && ok; ++k) {
@@ -141,7 +155,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_gemm_tma(const __grid_constant_
         if (!mbar_wait(sa(&tempty[b]), bph ^ 1u, abort_v)) { give_up(); ok = false; break; }
         asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
         const uint32_t d = tmem + (uint32_t)(b * P.acc_stride);
-        const TmaGemm& g = P.g[t >= P.tiles0];
+        const TmaGemm& g = P.g[!ONE && t >= P.tiles0];
         const uint32_t idesc = idesc_bf16(kBM, g.bn);
         const int nk = (g.K + kBK - 1) / kBK;
         for (int k = 0; k < nk; ++k) {
@@ -171,6 +185,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_gemm_tma(const __grid_constant_
   } else {
     const int q = warp & 3;            // tensor-memory lane quarter this warp may read
     const int half = (warp - 2) >> 2;  // which of the two warps of that quarter
+    const TmaGemm g0 = P.g[0];  // in registers: through P they are read again after every store
     int it = 0;
     for (int t = blockIdx.x; t < ntiles; t += gridDim.x, ++it) {
       const int b = it & 1;
@@ -178,13 +193,12 @@ __global__ void __launch_bounds__(kThreads, 1) k_gemm_tma(const __grid_constant_
       if (!mbar_wait(sa(&tfull[b]), bph, abort_v)) { give_up(); break; }
       asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
       const uint32_t tbase = tmem + ((uint32_t)(q * 32) << 16) + (uint32_t)(b * P.acc_stride);
-      const int p = t >= P.tiles0;
-      const TmaGemm& g = P.g[p];
-      const int tp = p ? t - P.tiles0 : t, n0 = tp % g.nt * g.bn;
-      const int N = min(g.N, n0 + g.bn);
-      const size_t row = (size_t)(tp / g.nt) * kBM + (size_t)q * 32 + lane;
-#pragma unroll 1
-      for (int c0 = n0 + 32 * half; c0 < N; c0 += 64) {
+      const int p = !ONE && t >= P.tiles0;
+      const TmaGemm& g = ONE ? g0 : P.g[p];
+      const int tp = p ? t - P.tiles0 : t, n0 = ONE ? 0 : tp % g.nt * g.bn;
+      const int N = ONE ? g.N : min(g.N, n0 + g.bn);
+      const size_t row = (size_t)(ONE ? tp : tp / g.nt) * kBM + (size_t)q * 32 + lane;
+      auto columns = [&](int c0) {
         uint32_t r[32];
         TMEM_LD32X32(tbase + (uint32_t)(c0 - n0), r);
         asm volatile("tcgen05.wait::ld.sync.aligned;\n" ::: "memory");
@@ -203,7 +217,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_gemm_tma(const __grid_constant_
           for (int j = 0; j < 8; ++j)
             if (4 * j < ncol) dst[j] = make_float4(v[4 * j], v[4 * j + 1], v[4 * j + 2], v[4 * j + 3]);
         }
-        if (g.z) {
+        if (!ONE && g.z) {
           const float4* zs = reinterpret_cast<const float4*>(g.z + o);
 #pragma unroll
           for (int j = 0; j < 8; ++j)
@@ -215,18 +229,21 @@ __global__ void __launch_bounds__(kThreads, 1) k_gemm_tma(const __grid_constant_
               v[4 * j + 3] *= gelu_grad(z.w);
             }
         }
-        if (g.out_bf16 || g.out_t) {
+        if (ONE && g.out_bf16) {
+          uint4* dst = reinterpret_cast<uint4*>(g.out_bf16 + o);
+#pragma unroll
+          for (int j = 0; j < 4; ++j) {
+            if (8 * j >= ncol) break;
+            uint32_t w[4];
+#pragma unroll
+            for (int k = 0; k < 4; ++k) w[k] = pack(g, c0 + 8 * j + 2 * k, v[8 * j + 2 * k], v[8 * j + 2 * k + 1]);
+            dst[j] = make_uint4(w[0], w[1], w[2], w[3]);
+          }
+        }
+        if (!ONE && (g.out_bf16 || g.out_t)) {
           uint32_t w[16];
 #pragma unroll
-          for (int k = 0; k < 16; ++k) {
-            float x0 = v[2 * k], x1 = v[2 * k + 1];
-            if (g.gelu) {
-              if (c0 + 2 * k < g.n_valid) x0 = gelu_f(x0);
-              if (c0 + 2 * k + 1 < g.n_valid) x1 = gelu_f(x1);
-            }
-            const __nv_bfloat162 p2 = __floats2bfloat162_rn(x0, x1);
-            w[k] = *reinterpret_cast<const uint32_t*>(&p2);
-          }
+          for (int k = 0; k < 16; ++k) w[k] = pack(g, c0 + 2 * k, v[2 * k], v[2 * k + 1]);
           if (g.out_bf16) {
             uint4* dst = reinterpret_cast<uint4*>(g.out_bf16 + o);
 #pragma unroll
@@ -241,6 +258,12 @@ __global__ void __launch_bounds__(kThreads, 1) k_gemm_tma(const __grid_constant_
               if (j < ncol) dst[(size_t)j * g.ldt] = (uint16_t)(w[j >> 1] >> (16 * (j & 1)));
           }
         }
+      };
+      if constexpr (ONE) {
+        for (int c0 = n0 + 32 * half; c0 < N; c0 += 64) columns(c0);
+      } else {
+#pragma unroll 1
+        for (int c0 = n0 + 32 * half; c0 < N; c0 += 64) columns(c0);
       }
       asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
       mbar_arrive(sa(&tempty[b]));
@@ -288,7 +311,9 @@ cudaError_t gemm_tma_prepare() {
   cudaError_t e = cudaGetDevice(&dev);
   if (e == cudaSuccess) e = cudaDeviceGetAttribute(&g_sms, cudaDevAttrMultiProcessorCount, dev);
   if (e == cudaSuccess)
-    e = cudaFuncSetAttribute(k_gemm_tma, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)tma_smem(256));
+    e = cudaFuncSetAttribute(k_gemm_tma<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)tma_smem(256));
+  if (e == cudaSuccess)
+    e = cudaFuncSetAttribute(k_gemm_tma<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)tma_smem(256));
   return e;
 }
 
@@ -330,7 +355,8 @@ cudaError_t launch_gemm_tma(const GemmArgs* a, int n, cudaStream_t st) {
   P.err = a[0].err;
   const int grid = P.tiles < g_sms ? P.tiles : g_sms;
   if (grid == 0) return cudaSuccess;
-  k_gemm_tma<<<grid, kThreads, tma_smem(wide), st>>>(P);
+  const bool one = n == 1 && P.g[0].nt == 1 && !a[0].z && !a[0].out_t;
+  (one ? k_gemm_tma<true> : k_gemm_tma<false>)<<<grid, kThreads, tma_smem(wide), st>>>(P);
   return cudaGetLastError();
 }
 
