@@ -1020,7 +1020,7 @@ static felis_status diag_now(felis_handle* h, double* twiss_dev, double* bf_dev)
   {
     KernelScope ks(h, FELIS_KERNEL_REDUCE);
     launch_diag_finalize(h->d_part, (int)h->tiles.size(), h->diag_stride, h->p.num_species, h->p.num_harmony,
-                         h->d_tiles, h->d_l1, h->l1_blocks, twiss_dev, bf_dev, h->st);
+                         h->d_tiles, h->d_l1, h->l1_blocks, twiss_dev, bf_dev, nullptr, 0, 0, nullptr, h->st);
   }
   CK(cudaGetLastError());
   return FELIS_OK;
@@ -1281,8 +1281,8 @@ static felis_status step_impl(felis_handle* h, int it) {
     {
       KernelScope ks(h, FELIS_KERNEL_REDUCE);
       launch_diag_finalize(h->d_part, (int)h->tiles.size(), h->diag_stride, ns, H, h->d_tiles, h->d_l1, h->l1_blocks,
-                           h->d_hist_t + (size_t)(it + 1) * 6 * ns, h->d_hist_b + (size_t)(it + 1) * 2 * H, h->st);
-      launch_sum_planes(h->d_planes, H, h->p.slice_n, shift ? 1 : 0, h->d_hist_e + (size_t)(it + 1) * 2 * H, h->st);
+                           h->d_hist_t + (size_t)(it + 1) * 6 * ns, h->d_hist_b + (size_t)(it + 1) * 2 * H,
+                           h->d_planes, h->p.slice_n, shift ? 1 : 0, h->d_hist_e + (size_t)(it + 1) * 2 * H, h->st);
       h->launches[FELIS_KERNEL_REDUCE] += 1;
     }
     CK(cudaGetLastError());

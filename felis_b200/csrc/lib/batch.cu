@@ -653,7 +653,14 @@ felis_status ensure_launch(felis_batch* b) {
   b->push_smem = (int)batch_push_smem(b->nsrc_max, b->LF_max, b->nr_max, std::min(b->N_max, b->push_box));
   const int push_max = (int)batch_push_smem(b->nsrc_max, b->LF_max, b->nr_max, std::min(b->N_max, 6144));
   b->push_threads = (int)std::max<int64_t>(m, 1) * kPushThreads;
-  if (batch_set_smem(b->H_max, b->L_max, b->adi_smem_max, push_max) != cudaSuccess)
+  // a wide CTA holds somewhat more static shared memory: where that does not
+  // fit, 128 threads
+  if (m > 1 && batch_set_smem(b->H_max, b->L_max, true, b->adi_smem_max, push_max) != cudaSuccess) {
+    cudaGetLastError();
+    b->push_threads = kPushThreads;
+  }
+  if (b->push_threads == kPushThreads &&
+      batch_set_smem(b->H_max, b->L_max, false, b->adi_smem_max, push_max) != cudaSuccess)
     return bfail(b, FELIS_UNSUPPORTED, "shared memory of the ensemble launches exceeds the device limit");
   return FELIS_OK;
 }

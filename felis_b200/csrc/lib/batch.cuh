@@ -131,7 +131,7 @@ size_t batch_adi_smem(int nx, int ny, int src_cells);
 // Shared memory of the push launch with room for the accumulators of
 // `box_cells` source cells of every source plane.
 size_t batch_push_smem(int nsrc_max, int LF_max, int nr_max, int box_cells);
-cudaError_t batch_set_smem(int H, int L, int adi_bytes, int push_bytes);
+cudaError_t batch_set_smem(int H, int L, bool wide, int adi_bytes, int push_bytes);
 // CTAs of each kernel that fit on one SM with this shape.
 int batch_resident_adi(int threads, int smem_bytes);
 

@@ -517,60 +517,80 @@ __global__ void __launch_bounds__(256, HM == 1 ? 4 : 3) k_particles(const __grid
 
 // Level 1: block b sums tiles [b*per, (b+1)*per) of every quantity in a
 // fixed order: 7 twiss sums per species, then the 2H+1 bFactor sums.
-__global__ void __launch_bounds__(256) k_diag_level1(const double* part, int ntiles, int stride, int nspecies,
-                                                     int H, const int4* tiles, int per, double* out) {
-  __shared__ double red[8];
-  const int t0 = blockIdx.x * per, t1 = min(ntiles, t0 + per);
-  const int nq = 7 * nspecies + 2 * H + 1;
-  double* o = out + (size_t)blockIdx.x * nq;
-  for (int sp = 0; sp < nspecies; ++sp)
-    for (int k = 0; k < 7; ++k) {
-      double v = 0.0;
-      for (int t = t0 + threadIdx.x; t < t1; t += blockDim.x)
-        if (tiles[t].x == sp) v += part[(size_t)t * stride + k];
-      const double r = block_sum(v, red);
-      if (threadIdx.x == 0) o[7 * sp + k] = r;
+// The sums of nq quantities over rows [r0, r1) by a CTA of 256 threads, each as
+// block_sum forms it over its rows (a thread's rows in order, warp trees, the
+// warps in order), eight quantities at a time with their loads in flight
+// together and one barrier for all: at one slice a step's reductions took
+// 0.0189 ms with two barriers and a load's latency per quantity and a launch of
+// their own for the planes, 0.0127 with this.
+// value(row, q, &v) adds row's share of quantity q.  Thread q < nq returns its total.
+constexpr int kMaxSums = 7 * FELIS_MAX_SPECIES + 2 * FELIS_MAX_HARMONY + 1;
+template <class F>
+__device__ __forceinline__ double row_sums(int nq, int r0, int r1, F value) {
+  static_assert(kMaxSums <= 256, "a thread per quantity");
+  __shared__ double part[8][kMaxSums];
+  const int w = threadIdx.x >> 5, ln = threadIdx.x & 31;
+  for (int q0 = 0; q0 < nq; q0 += 8) {
+    double v[8] = {};
+    for (int r = r0 + threadIdx.x; r < r1; r += 256)
+#pragma unroll
+      for (int u = 0; u < 8; ++u)
+        if (q0 + u < nq) value(r, q0 + u, v[u]);
+#pragma unroll
+    for (int u = 0; u < 8; ++u) {
+      if (q0 + u >= nq) break;
+      for (int o = 16; o > 0; o >>= 1) v[u] += __shfl_down_sync(0xffffffffu, v[u], o);
+      if (ln == 0) part[w][q0 + u] = v[u];
     }
-  for (int k = 0; k < 2 * H + 1; ++k) {
-    double v = 0.0;
-    for (int t = t0 + threadIdx.x; t < t1; t += blockDim.x) v += part[(size_t)t * stride + 7 + k];
-    const double r = block_sum(v, red);
-    if (threadIdx.x == 0) o[7 * nspecies + k] = r;
-  }
-}
-
-// Level 2: one block adds the level-1 rows in order and finishes
-// twiss.cpp:177-192 and saveFile.cpp:166 (b / totalN).
-__global__ void __launch_bounds__(256) k_diag_level2(const double* l1, int nblocks, int nspecies, int H,
-                                                     double* twiss, double* bf) {
-  __shared__ double red[8];
-  const int nq = 7 * nspecies + 2 * H + 1;
-  __shared__ double tot[7 * FELIS_MAX_SPECIES + 2 * FELIS_MAX_HARMONY + 1];
-  for (int k = 0; k < nq; ++k) {
-    double v = 0.0;
-    for (int b = threadIdx.x; b < nblocks; b += blockDim.x) v += l1[(size_t)b * nq + k];
-    const double r = block_sum(v, red);
-    if (threadIdx.x == 0) tot[k] = r;
   }
   __syncthreads();
-  if (threadIdx.x == 0) {
-    for (int sp = 0; sp < nspecies; ++sp) {
-      const double* acc = tot + 7 * sp;
-      double* o = twiss + 6 * sp;
-      for (int k = 0; k < 6; ++k) o[k] = 0.0;
-      const double cnt = acc[6];
-      if (cnt > 0.0) {
-        const double avgX2 = acc[0] / cnt, avgY2 = acc[1] / cnt;
-        const double avgXP = acc[2] / cnt, avgYP = acc[3] / cnt;
-        const double avgCX = acc[4] / cnt, avgCY = acc[5] / cnt;
-        const double ex = sqrt(avgX2 * avgXP - avgCX * avgCX), ey = sqrt(avgY2 * avgYP - avgCY * avgCY);
-        o[0] = ex; o[1] = avgX2 / ex; o[2] = -avgCX / ex;
-        o[3] = ey; o[4] = avgY2 / ey; o[5] = -avgCY / ey;
-      }
-    }
-    const double wsum = tot[7 * nspecies + 2 * H];
-    for (int k = 0; k < 2 * H; ++k) bf[k] = tot[7 * nspecies + k] / wsum;
+  double t = 0.0;
+  if ((int)threadIdx.x < nq)
+    for (int k = 0; k < 8; ++k) t += part[k][threadIdx.x];
+  return t;
+}
+
+// Blocks [0, l1): the beam sums of `per` tiles each; blocks from l1 on: the sum
+// of a plane's energies over the slices (launch_sum_planes, in the same launch).
+__global__ void __launch_bounds__(256) k_diag_level1(const double* part, int ntiles, int stride, int nspecies,
+                                                     int H, const int4* tiles, int per, int l1, double* out,
+                                                     const double* planes, int S, int last, double* out_planes) {
+  if ((int)blockIdx.x >= l1) {
+    const int hp = blockIdx.x - l1;
+    const double t = row_sums(1, 0, last, [&](int s, int, double& v) { v += planes[(size_t)hp * S + s]; });
+    if (threadIdx.x == 0) out_planes[hp] = t;
+    return;
   }
+  const int t0 = blockIdx.x * per, t1 = min(ntiles, t0 + per), nb = 7 * nspecies, nq = nb + 2 * H + 1;
+  const double r = row_sums(nq, t0, t1, [&](int t, int q, double& v) {
+    if (q >= nb) v += part[(size_t)t * stride + 7 + (q - nb)];
+    else if (tiles[t].x == q / 7) v += part[(size_t)t * stride + q % 7];
+  });
+  if ((int)threadIdx.x < nq) out[(size_t)blockIdx.x * nq + threadIdx.x] = r;
+}
+
+__global__ void __launch_bounds__(256) k_diag_level2(const double* l1, int nblocks, int nspecies, int H,
+                                                     double* twiss, double* bf) {
+  const int nq = 7 * nspecies + 2 * H + 1, tid = threadIdx.x;
+  __shared__ double tot[kMaxSums];
+  const double r = row_sums(nq, 0, nblocks, [&](int b, int q, double& v) { v += l1[(size_t)b * nq + q]; });
+  if (tid < nq) tot[tid] = r;
+  __syncthreads();
+  // species by plane, a warp apart; the bunching factors by the last warps
+  for (int k = tid >> 5; k < 2 * nspecies && (tid & 31) == 0; k += 4) {
+    if (tid >= 128) break;
+    const double* acc = tot + 7 * (k >> 1);
+    double* o = twiss + 6 * (k >> 1) + 3 * (k & 1);
+    const int y = k & 1;
+    o[0] = o[1] = o[2] = 0.0;
+    const double cnt = acc[6];
+    if (cnt > 0.0) {
+      const double a2 = acc[y] / cnt, ap = acc[2 + y] / cnt, ac = acc[4 + y] / cnt;
+      const double e = sqrt(a2 * ap - ac * ac);
+      o[0] = e; o[1] = a2 / e; o[2] = -ac / e;
+    }
+  }
+  if (tid >= 128 && tid - 128 < 2 * H) bf[tid - 128] = tot[7 * nspecies + tid - 128] / tot[7 * nspecies + 2 * H];
 }
 
 }  // namespace
@@ -595,9 +615,11 @@ void launch_particles(const ParticleLaunch& a, cudaStream_t st) {
 }
 
 void launch_diag_finalize(const double* partials, int ntiles, int stride, int nspecies, int H, const int4* tiles,
-                          double* l1, int l1_blocks, double* out_twiss, double* out_bf, cudaStream_t st) {
+                          double* l1, int l1_blocks, double* out_twiss, double* out_bf, const double* planes, int S,
+                          int skip_last, double* out_planes, cudaStream_t st) {
   const int per = (ntiles + l1_blocks - 1) / l1_blocks;
-  k_diag_level1<<<l1_blocks, 256, 0, st>>>(partials, ntiles, stride, nspecies, H, tiles, per, l1);
+  k_diag_level1<<<l1_blocks + (planes ? 2 * H : 0), 256, 0, st>>>(partials, ntiles, stride, nspecies, H, tiles, per,
+                                                                  l1_blocks, l1, planes, S, S - skip_last, out_planes);
   k_diag_level2<<<1, 256, 0, st>>>(l1, l1_blocks, nspecies, H, out_twiss, out_bf);
 }
 
