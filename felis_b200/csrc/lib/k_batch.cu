@@ -1223,6 +1223,9 @@ __global__ void __launch_bounds__(WIDE ? PushWide<HM>::value : kPushThreads, WID
     }
   };
   if (push && !dep) {
+    // 128 threads of a wide CTA read what all of them have pushed; a thread of
+    // a CTA of 128 reads its own particles only
+    if (WIDE) __syncthreads();
     if (!WIDE || tid < kPushThreads)
       for (int q = tid; q < P; q += snt) {
         const int64_t n = p0 + q;
