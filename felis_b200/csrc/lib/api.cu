@@ -609,7 +609,7 @@ felis_status relayout(felis_handle* h, const std::vector<int64_t>& new_counts_pe
   for (int k = 0; k < h->p.num_harmony; ++k) neven += (h->p.harmony[k] % 2 == 0);
   if (!deposit_plan(h->p.num_harmony, neven, h->p.scl_mode, h->p.scf_mode, h->p.nr, (size_t)dev_smem, &h->dep_plan))
     return fail(h, FELIS_UNSUPPORTED, "deposit buffers do not fit in shared memory");
-  deposit_set_smem(h->dep_plan.smem);
+  CK(deposit_set_smem(h->dep_plan.smem));
   invalidate_particles(h);
   return FELIS_OK;
 }
@@ -790,14 +790,16 @@ felis_status felis_create(const felis_params* p, felis_handle** out) {
     int dev_smem = 0;
     cudaDeviceGetAttribute(&dev_smem, cudaDevAttrMaxSharedMemoryPerBlockOptin, h->device);
     if (st == FELIS_OK && (int)smem <= dev_smem - 1024) {
-      adi_set_smem(smem);
+      if (adi_set_smem(smem) != cudaSuccess) bail(FELIS_CUDA_ERROR, "ADI shared memory");
     } else if (st == FELIS_OK) {
       // plane larger than shared memory: swept in tiles, one scratch plane per
       // CTA of a persistent grid
       h->adi_big_grid = std::min(S * H * 2, h->sms * 2);
       if (cudaMalloc(&h->adi_scratch, (size_t)h->adi_big_grid * nx * ny * sizeof(double2)) != cudaSuccess)
         bail(FELIS_CUDA_ERROR, "ADI scratch allocation failed");
-      adi_big_set_smem(adi_big_smem_bytes(nx, ny));
+      // (grids wider than 256 points are refused below)
+      if (std::max(nx, ny) <= 256 && adi_big_set_smem(adi_big_smem_bytes(nx, ny)) != cudaSuccess)
+        bail(FELIS_CUDA_ERROR, "ADI shared memory");
     }
     if (st == FELIS_OK && std::max(nx, ny) > 256) bail(FELIS_UNSUPPORTED, "grid wider than 256 points");
   }

@@ -29,6 +29,23 @@ inline double phase_shift_of(int n, const double* z, const double* phase, int it
   return d;
 }
 
+// Lets launches of a kernel take `bytes` of dynamic shared memory.  The limit
+// belongs to the kernel on a device, not to the handle or ensemble that asks:
+// it is set to all that the device gives beside the kernel's static part, so
+// that whichever asks last takes nothing from the others.  cudaErrorInvalidValue
+// when `bytes` do not fit.
+inline cudaError_t allow_smem(const void* kernel, size_t bytes) {
+  cudaFuncAttributes at{};
+  int dev = 0, most = 0;
+  cudaError_t e = cudaGetDevice(&dev);
+  if (e == cudaSuccess) e = cudaDeviceGetAttribute(&most, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
+  if (e == cudaSuccess) e = cudaFuncGetAttributes(&at, kernel);
+  if (e != cudaSuccess) return e;
+  const int room = most - (int)at.sharedSizeBytes;
+  if (room < 0 || bytes > (size_t)room) return cudaErrorInvalidValue;
+  return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, room);
+}
+
 // ---- complex arithmetic ----------------------------------------------------
 // Same operand order as std::complex<double> in the reference; division is
 // the limited-range, reciprocal expansion its -ffast-math build selects.

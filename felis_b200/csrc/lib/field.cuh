@@ -67,14 +67,15 @@ void launch_deposit(const DepositLaunch& a, size_t smem, cudaStream_t st);
 // Multiplier and pivot of every point and mode of the radial Ez solve with
 // the coefficient A (DepositLaunch::A): L * F <= 16 modes.
 void launch_radial_elimination(double A, int L, int F, int nr, const double* logtab, double2* out, cudaStream_t st);
-void deposit_set_smem(size_t bytes);
-void adi_set_smem(size_t bytes);
+// The shared memory that launches may take (allow_smem).
+cudaError_t deposit_set_smem(size_t bytes);
+cudaError_t adi_set_smem(size_t bytes);
 void launch_adi(const AdiLaunch& a, cudaStream_t st);
 size_t adi_smem_bytes(int nx, int ny, int nxp);
 // Planes larger than shared memory: `grid` CTAs, each with one scratch plane.
 void launch_adi_big(AdiLaunch a, int grid, cudaStream_t st);
 size_t adi_big_smem_bytes(int nx, int ny);
-void adi_big_set_smem(size_t bytes);
+cudaError_t adi_big_set_smem(size_t bytes);
 void launch_energy(const DevGeom& G, const double2* U, int ring_base, double* out_planes, cudaStream_t st);
 void launch_sum_planes(const double* planes, int H, int S, int skip_last, double* out, cudaStream_t st);
 

@@ -1583,10 +1583,8 @@ size_t batch_push_smem(int nsrc_max, int LF_max, int nr_max, int box_cells) {
 }
 
 cudaError_t batch_set_smem(int H, int L, bool wide, int adi_bytes, int push_bytes) {
-  cudaError_t e = cudaFuncSetAttribute(k_batch_adi, cudaFuncAttributeMaxDynamicSharedMemorySize, adi_bytes);
-  if (e == cudaSuccess)
-    e = cudaFuncSetAttribute(push_kernel(H, L, wide), cudaFuncAttributeMaxDynamicSharedMemorySize, push_bytes);
-  return e;
+  const cudaError_t e = allow_smem((const void*)k_batch_adi, (size_t)adi_bytes);
+  return e == cudaSuccess ? allow_smem((const void*)push_kernel(H, L, wide), (size_t)push_bytes) : e;
 }
 
 int batch_resident_adi(int threads, int smem_bytes) {

@@ -568,8 +568,6 @@ void launch_radial_elimination(double A, int L, int F, int nr, const double* log
   k_radial_elimination<<<1, 32, 0, st>>>(A, L * F, F, nr, logtab, out);
 }
 
-void deposit_set_smem(size_t bytes) {
-  cudaFuncSetAttribute(k_deposit, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
-}
+cudaError_t deposit_set_smem(size_t bytes) { return allow_smem((const void*)k_deposit, bytes); }
 
 }  // namespace felis

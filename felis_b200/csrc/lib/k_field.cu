@@ -408,9 +408,7 @@ __global__ void __launch_bounds__(256) k_sum_planes(const double* planes, int S,
 
 }  // namespace
 
-void adi_set_smem(size_t bytes) {
-  cudaFuncSetAttribute(k_adi, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
-}
+cudaError_t adi_set_smem(size_t bytes) { return allow_smem((const void*)k_adi, bytes); }
 
 size_t adi_smem_bytes(int nx, int ny, int nxp) {
   return (size_t)ny * nxp * sizeof(double2) + (size_t)4 * (nx + ny) * sizeof(double2) + (size_t)3 * (nx + ny) * sizeof(double);
@@ -435,9 +433,7 @@ static size_t adi_tile_cells(int nx, int ny) {
 
 size_t adi_big_smem_bytes(int nx, int ny) { return adi_tile_cells(nx, ny) * sizeof(double2) + (size_t)88 * (nx + ny); }
 
-void adi_big_set_smem(size_t bytes) {
-  cudaFuncSetAttribute(k_adi_big, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
-}
+cudaError_t adi_big_set_smem(size_t bytes) { return allow_smem((const void*)k_adi_big, bytes); }
 
 void launch_adi_big(AdiLaunch a, int grid, cudaStream_t st) {
   a.tile_cells = (int)adi_tile_cells(a.G.nx, a.G.ny);
