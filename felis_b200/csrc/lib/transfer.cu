@@ -18,6 +18,28 @@
 
 namespace felis {
 
+namespace {
+
+// `device` current in this thread (the events are made on it and belong to it),
+// and the caller's device current again at the end.
+struct OnDevice {
+  int was = -1;
+  cudaError_t status;
+  explicit OnDevice(int device) {
+    status = cudaGetDevice(&was);
+    if (status != cudaSuccess) was = -1;
+    else if (was == device) was = -1;
+    else status = cudaSetDevice(device);
+  }
+  ~OnDevice() {
+    if (was >= 0) cudaSetDevice(was);
+  }
+  OnDevice(const OnDevice&) = delete;
+  OnDevice& operator=(const OnDevice&) = delete;
+};
+
+}  // namespace
+
 HostStage::~HostStage() {
   for (auto& t : ev_)
     for (cudaEvent_t e : t)
@@ -49,6 +71,8 @@ cudaError_t HostStage::run(const CopyPart* parts, int nparts, Mode mode, int dev
       total += n;
     }
   if (!total) return cudaSuccess;
+  const OnDevice here(device);
+  if (here.status != cudaSuccess) return here.status;
   if (!pinned_ && total < kChunk && mode != kDownWiden) {
     // too little to page-lock memory for (2 ms)
     for (const CopyPart& c : chunks) {
@@ -88,7 +112,7 @@ cudaError_t HostStage::run(const CopyPart* parts, int nparts, Mode mode, int dev
         for (size_t k = 0; k < c.bytes / sizeof(float); ++k) d[k] = f[k];
       }
     };
-    if (fail(cudaSetDevice(device))) return;
+    if (t && fail(cudaSetDevice(device))) return;
     int s = 0;
     for (size_t i; status == cudaSuccess && (i = next++) < chunks.size(); s = (s + 1) % kSlots) {
       if (busy[s]) finish(s);

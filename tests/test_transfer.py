@@ -1,0 +1,60 @@
+"""The staged copies between device and host (HostStage) on the CPU: the source
+file compiled against a host stand-in for the few runtime calls it makes, with
+two devices, streams and events that belong to one of them, and page-locked
+memory that can run out."""
+import ctypes as C
+import os
+import subprocess
+
+import numpy as np
+import pytest
+
+ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+DOWN, WIDEN, UP = 0, 1, 2
+MB = 1 << 20
+
+
+@pytest.fixture(scope="module")
+def lib(tmp_path_factory):
+    fake = os.path.join(ROOT, "tests", "host_cuda")
+    src = os.path.join(ROOT, "felis_b200", "csrc", "lib")
+    out = str(tmp_path_factory.mktemp("transfer") / "transfer_host.so")
+    subprocess.run(["g++", "-std=c++17", "-O1", "-shared", "-fPIC", "-pthread", f"-I{fake}", f"-I{src}", "-x", "c++",
+                    os.path.join(src, "transfer.cu"), os.path.join(fake, "transfer_calls.cpp"), "-o", out], check=True)
+    so = C.CDLL(out)
+    so.stage_new.restype = C.c_void_p
+    so.stage_free.argtypes = [C.c_void_p]
+    p, n = C.c_void_p, C.c_size_t
+    so.stage_copy.argtypes = [p, C.c_int, C.c_int, C.c_int, p, p, n, p, p, n, C.POINTER(C.c_int)]
+    return so
+
+
+def _copy(lib, stage, how, words, device=0, current=0, split=0.3):
+    """One call over `words` 32-bit values in two parts: (status, device
+    afterwards, whether every value arrived)."""
+    a = np.random.default_rng(words).standard_normal(words).astype(np.float32)
+    b = np.zeros(words, np.float64 if how == WIDEN else np.float32)
+    k, after = int(words * split), C.c_int(-1)
+    st = lib.stage_copy(stage, how, device, current, a.ctypes.data, b.ctypes.data, 4 * k, a[k:].ctypes.data,
+                        b[k:].ctypes.data, 4 * (words - k), C.byref(after))
+    return st, after.value, np.array_equal(a, b)
+
+
+@pytest.fixture
+def stage(lib):
+    s = lib.stage_new()
+    yield s
+    lib.stage_free(s)
+    assert lib.host_live() == 0
+
+
+@pytest.mark.parametrize("how", [DOWN, WIDEN, UP])
+@pytest.mark.parametrize("words", [100, 100_001, 5 * MB, 20 * MB + 3])
+def test_a_handle_of_another_device(lib, stage, how, words):
+    """Copies work, and leave the caller's device, whichever is current."""
+    for device, current in ((1, 0), (1, 1), (0, 1), (1, 0)):
+        s = lib.stage_new()
+        for _ in range(2):
+            assert _copy(lib, s, how, words, device, current) == (0, current, True)
+        lib.stage_free(s)
+    assert _copy(lib, stage, how, words, 1, 0) == (0, 0, True)
