@@ -12,8 +12,9 @@ struct CopyPart {
   size_t bytes;  // at the source (a multiple of 4)
 };
 
-// Page-locked slots of one handle, ensemble or network, made at its first copy
-// and freed with it (16 MB at most).  One call at a time, like its owner.
+// Page-locked slots of one handle, ensemble or network, made when its copies
+// have come to kLockAfter bytes and freed with it (16 MB at most).  One call at
+// a time, like its owner.
 class HostStage {
  public:
   HostStage() = default;
@@ -29,9 +30,12 @@ class HostStage {
  private:
   static constexpr int kThreads = 8, kSlots = 2;
   static constexpr size_t kChunk = (size_t)1 << 20;
+  // bytes at the destination for which plain copies cost what the slots do
+  static constexpr size_t kLockAfter = (size_t)64 << 20;
   char* pinned_ = nullptr;  // [threads_][kSlots][kChunk]
   cudaEvent_t ev_[kThreads][kSlots] = {};
   int threads_ = 0;
+  size_t moved_ = 0;  // bytes at the destination so far
   cudaError_t reserve(int threads);
   enum Mode { kDown, kDownWiden, kUp };
   cudaError_t run(const CopyPart* parts, int nparts, Mode mode, int device, cudaStream_t st);

@@ -58,3 +58,21 @@ def test_a_handle_of_another_device(lib, stage, how, words):
             assert _copy(lib, s, how, words, device, current) == (0, current, True)
         lib.stage_free(s)
     assert _copy(lib, stage, how, words, 1, 0) == (0, 0, True)
+
+
+@pytest.mark.parametrize("how", [DOWN, WIDEN, UP])
+def test_small_copies_lock_no_pages(lib, stage, how):
+    """Slots cost milliseconds to make: an object has them only once its copies
+    have come to 64 MB at the destination, in one call or in many."""
+    per = MB // (2 if how == WIDEN else 1)  # 4 MB at the destination
+    before = lib.host_allocations()
+    for _ in range(15):
+        assert _copy(lib, stage, how, per) == (0, 0, True)
+    assert lib.host_allocations() == before and lib.host_live() == 0
+    for _ in range(3):
+        assert _copy(lib, stage, how, per) == (0, 0, True)
+    assert lib.host_live() == 1
+    one = lib.stage_new()
+    assert _copy(lib, one, how, 16 * per) == (0, 0, True)
+    assert lib.host_live() == 2
+    lib.stage_free(one)
