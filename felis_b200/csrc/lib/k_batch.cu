@@ -320,11 +320,11 @@ __global__ void __launch_bounds__(1024) k_batch_adi(BatchLaunch a) {
   }
   const bool src = Sc != nullptr;
   cp_async_wait_all();
+  __syncthreads();  // the staged cells of all threads, and tbar made before any thread waits on it
   if (tb_bulk && !bar_wait0(smem_u32(&tbar), kBulkWaitTries)) {
     atomicOr(I.err + ERR_TIMEOUT, 1);
     bar_wait0(smem_u32(&tbar), kBulkWaitTries);  // once more for the copy in flight
   }
-  __syncthreads();
   const float2 zero = make_float2(0.f, 0.f);
   const int* K8 = I.adi_k[h];
   const int kx0 = K8[0], kx1 = K8[1], ky0 = K8[2], ky1 = K8[3], gx = K8[4], qx = K8[5], gy = K8[6], qy = K8[7];
