@@ -578,10 +578,10 @@ felis_status relayout(felis_handle* h, const std::vector<int64_t>& new_counts_pe
   if (h->d_part) cudaFree(h->d_part);
   h->d_soff = nullptr; h->d_tiles = nullptr; h->d_part = nullptr;
   CK(cudaMalloc(&h->d_soff, soff.size() * sizeof(int64_t)));
-  CK(cudaMemcpy(h->d_soff, soff.data(), soff.size() * sizeof(int64_t), cudaMemcpyHostToDevice));
+  CK(to_device(h->d_soff, soff.data(), soff.size() * sizeof(int64_t), h->st));
   CK(cudaMalloc(&h->d_tiles, std::max<size_t>(h->tiles.size(), 1) * sizeof(int4)));
   if (!h->tiles.empty())
-    CK(cudaMemcpy(h->d_tiles, h->tiles.data(), h->tiles.size() * sizeof(int4), cudaMemcpyHostToDevice));
+    CK(to_device(h->d_tiles, h->tiles.data(), h->tiles.size() * sizeof(int4), h->st));
   CK(cudaMalloc(&h->d_part, std::max<size_t>(h->tiles.size(), 1) * h->diag_stride * sizeof(double)));
   // deposit records
   if (total > h->dep_cap) {
@@ -720,18 +720,18 @@ felis_status felis_create(const felis_params* p, felis_handle** out) {
   if (ce == cudaSuccess) ce = cudaMalloc(&h->Ez, ezn * sizeof(double2));
   if (ce == cudaSuccess) ce = cudaMemsetAsync(h->Ez, 0, ezn * sizeof(double2), h->st);
   if (ce == cudaSuccess) ce = cudaMalloc(&h->d_bessel, (size_t)p->bessel_rows * p->bessel_cols * sizeof(double));
-  if (ce == cudaSuccess) ce = cudaMemcpy(h->d_bessel, p->bessel, (size_t)p->bessel_rows * p->bessel_cols * sizeof(double), cudaMemcpyHostToDevice);
+  if (ce == cudaSuccess) ce = to_device(h->d_bessel, p->bessel, (size_t)p->bessel_rows * p->bessel_cols * sizeof(double), h->st);
   std::vector<double> wake(std::max(p->global_slice_n, 1), 0.0);
   h->p.wake_e = nullptr;
   h->p.abc_alpha = h->p.abc_alpha_p = h->p.abc_beta = h->p.abc_beta_p = nullptr;
   if (p->wake_e) std::copy(p->wake_e, p->wake_e + p->global_slice_n, wake.begin());
   if (ce == cudaSuccess) ce = cudaMalloc(&h->d_wake, wake.size() * sizeof(double));
-  if (ce == cudaSuccess) ce = cudaMemcpy(h->d_wake, wake.data(), wake.size() * sizeof(double), cudaMemcpyHostToDevice);
+  if (ce == cudaSuccess) ce = to_device(h->d_wake, wake.data(), wake.size() * sizeof(double), h->st);
   std::vector<double> logtab(p->nr, 0.0);
   for (int j = 1; j < p->nr; ++j) logtab[j] = log((j + 0.5) / (j - 0.5));
   if (ce == cudaSuccess) ce = cudaMalloc(&h->d_log, logtab.size() * sizeof(double));
   if (ce == cudaSuccess) ce = cudaMalloc(&h->d_radial, (size_t)p->scl_mode * p->scf_mode * p->nr * sizeof(double2));
-  if (ce == cudaSuccess) ce = cudaMemcpy(h->d_log, logtab.data(), logtab.size() * sizeof(double), cudaMemcpyHostToDevice);
+  if (ce == cudaSuccess) ce = to_device(h->d_log, logtab.data(), logtab.size() * sizeof(double), h->st);
   if (ce == cudaSuccess) ce = cudaMalloc(&h->d_planes, (size_t)H * 2 * S * sizeof(double));
   if (ce == cudaSuccess) ce = cudaMalloc(&h->d_planes2, (size_t)H * 2 * S * sizeof(double));
   h->hist_n = std::max(p->max_step, 1) + 1;
@@ -765,8 +765,8 @@ felis_status felis_create(const felis_params* p, felis_handle** out) {
       cd* dc = nullptr;
       double* dd = nullptr;
       if (cudaMalloc(&dc, cv.size() * sizeof(cd)) != cudaSuccess || cudaMalloc(&dd, dv.size() * sizeof(double)) != cudaSuccess ||
-          cudaMemcpy(dc, cv.data(), cv.size() * sizeof(cd), cudaMemcpyHostToDevice) != cudaSuccess ||
-          cudaMemcpy(dd, dv.data(), dv.size() * sizeof(double), cudaMemcpyHostToDevice) != cudaSuccess) {
+          to_device(dc, cv.data(), cv.size() * sizeof(cd), h->st) != cudaSuccess ||
+          to_device(dd, dv.data(), dv.size() * sizeof(double), h->st) != cudaSuccess) {
         bail(FELIS_CUDA_ERROR, "ADI table upload failed");
         break;
       }
@@ -782,7 +782,7 @@ felis_status felis_create(const felis_params* p, felis_handle** out) {
     }
     if (st == FELIS_OK) {
       if (cudaMalloc(&h->d_adi, H * sizeof(AdiTab)) != cudaSuccess ||
-          cudaMemcpy(h->d_adi, tabs.data(), H * sizeof(AdiTab), cudaMemcpyHostToDevice) != cudaSuccess)
+          to_device(h->d_adi, tabs.data(), H * sizeof(AdiTab), h->st) != cudaSuccess)
         bail(FELIS_CUDA_ERROR, "ADI table upload failed");
     }
     h->nxp = nx | 1;
@@ -880,7 +880,7 @@ felis_status felis_upload_particles(felis_handle* h, int32_t species, const doub
       const int sp = kept[k];
       const int64_t b = h->soff[(size_t)sp * (S + 1)], e = h->soff[(size_t)sp * (S + 1) + S];
       double* arrs[6] = {h->x, h->y, h->px, h->py, h->th, h->ga};
-      for (int q = 0; q < 6; ++q) CK(cudaMemcpy(arrs[q] + b, keep[k].data() + q * (e - b), (e - b) * sizeof(double), cudaMemcpyHostToDevice));
+      for (int q = 0; q < 6; ++q) CK(to_device(arrs[q] + b, keep[k].data() + q * (e - b), (e - b) * sizeof(double), h->st));
       h->uploaded[sp] = 1;
     }
   }
@@ -1457,8 +1457,8 @@ felis_status felis_set_first_planes(felis_handle* h, const double* in) {
   CK(cudaStreamSynchronize(h->st));
   for (int hh = 0; hh < H; ++hh)
     for (int pol = 0; pol < 2; ++pol)
-      CK(cudaMemcpy(h->U + field_plane(S, hh, pol, 0, h->ring_base) * N, in + 2 * ((size_t)(hh * 2 + pol) * N),
-                    N * sizeof(double2), cudaMemcpyHostToDevice));
+      CK(to_device(h->U + field_plane(S, hh, pol, 0, h->ring_base) * N, in + 2 * ((size_t)(hh * 2 + pol) * N),
+                    N * sizeof(double2), h->st));
   for (int k = 0; k < 2 * H; ++k)
     CK(cudaMemsetAsync(h->lit + field_plane(S, k >> 1, k & 1, 0, h->ring_base), 1, sizeof(int), h->st));
   h->diag_valid = false;

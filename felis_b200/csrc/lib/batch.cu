@@ -412,7 +412,7 @@ felis_status upload_inst_table(felis_batch* b) {
     D.bessel = I.d_bessel; D.wakeE = I.wake;
     D.adi_c = I.adi; D.part_e = I.part_e; D.part_b = I.part_b; D.err = I.err;
   }
-  BCK(cudaMemcpy(b->d_inst, h.data(), h.size() * sizeof(BInst), cudaMemcpyHostToDevice));
+  BCK(to_device(b->d_inst, h.data(), h.size() * sizeof(BInst), b->st));
   return FELIS_OK;
 }
 
@@ -612,8 +612,8 @@ felis_status prepare(felis_batch* b) {
   b->d_adi_work = b->d_push_work = nullptr;
   BCK(cudaMalloc(&b->d_adi_work, adi.size() * sizeof(int4)));
   BCK(cudaMalloc(&b->d_push_work, push.size() * sizeof(int4)));
-  BCK(cudaMemcpy(b->d_adi_work, adi.data(), adi.size() * sizeof(int4), cudaMemcpyHostToDevice));
-  BCK(cudaMemcpy(b->d_push_work, push.data(), push.size() * sizeof(int4), cudaMemcpyHostToDevice));
+  BCK(to_device(b->d_adi_work, adi.data(), adi.size() * sizeof(int4), b->st));
+  BCK(to_device(b->d_push_work, push.data(), push.size() * sizeof(int4), b->st));
   felis_status s = upload_inst_table(b);
   if (s != FELIS_OK) return s;
   b->layout_ready = true;
@@ -722,7 +722,7 @@ felis_status check_batch_err(felis_batch* b) {
     else if (b->h_err[ERR_RADIAL]) s = bfail(b, FELIS_UNSUPPORTED, "particle outside the radial Ez grid");
     else if (b->h_err[ERR_TIMEOUT]) s = bfail(b, FELIS_TIMEOUT, "a bounded device wait ran out");
     if (s != FELIS_OK) {
-      BCK(cudaMemset(I.err, 0, ERR_SLOTS * sizeof(int)));
+      BCK(cudaMemsetAsync(I.err, 0, ERR_SLOTS * sizeof(int), b->st));
       return s;
     }
   }
@@ -808,23 +808,23 @@ felis_status felis_batch_create(const felis_params* const* instances, int32_t n,
     if (e == cudaSuccess) e = cudaMalloc(&I.sbox, (size_t)S * sizeof(int4));
     if (e == cudaSuccess) {
       std::vector<int4> empty(S, make_int4(1, 0, 1, 0));
-      e = cudaMemcpy(I.sbox, empty.data(), S * sizeof(int4), cudaMemcpyHostToDevice);
+      e = to_device(I.sbox, empty.data(), S * sizeof(int4), b->st);
     }
     const size_t un = (size_t)H * 2 * S * N;
     if (e == cudaSuccess) e = cudaMalloc(&I.U, un * sizeof(float2));
-    if (e == cudaSuccess) e = cudaMemset(I.U, 0, un * sizeof(float2));
+    if (e == cudaSuccess) e = cudaMemsetAsync(I.U, 0, un * sizeof(float2), b->st);
     if (e == cudaSuccess) e = cudaMalloc(&I.lit, (size_t)H * 2 * S * sizeof(int));
-    if (e == cudaSuccess) e = cudaMemset(I.lit, 0, (size_t)H * 2 * S * sizeof(int));
+    if (e == cudaSuccess) e = cudaMemsetAsync(I.lit, 0, (size_t)H * 2 * S * sizeof(int), b->st);
     const size_t ezn = (size_t)p->scl_mode * S * p->scf_mode * p->nr;
     if (e == cudaSuccess) e = cudaMalloc(&I.Ez, ezn * sizeof(float2));
-    if (e == cudaSuccess) e = cudaMemset(I.Ez, 0, ezn * sizeof(float2));
+    if (e == cudaSuccess) e = cudaMemsetAsync(I.Ez, 0, ezn * sizeof(float2), b->st);
     std::vector<float> bf(I.bessel.begin(), I.bessel.end());
     if (e == cudaSuccess) e = cudaMalloc(&I.d_bessel, bf.size() * sizeof(float));
-    if (e == cudaSuccess) e = cudaMemcpy(I.d_bessel, bf.data(), bf.size() * sizeof(float), cudaMemcpyHostToDevice);
+    if (e == cudaSuccess) e = to_device(I.d_bessel, bf.data(), bf.size() * sizeof(float), b->st);
     std::vector<double> wk(std::max(p->global_slice_n, 1), 0.0);
     if (p->wake_e) std::copy(p->wake_e, p->wake_e + p->global_slice_n, wk.begin());
     if (e == cudaSuccess) e = cudaMalloc(&I.wake, wk.size() * sizeof(double));
-    if (e == cudaSuccess) e = cudaMemcpy(I.wake, wk.data(), wk.size() * sizeof(double), cudaMemcpyHostToDevice);
+    if (e == cudaSuccess) e = to_device(I.wake, wk.data(), wk.size() * sizeof(double), b->st);
     adi_chunks(p->nx - 2, I.cx);
     adi_chunks(p->ny - 2, I.cy);
     std::vector<float2> tabs;
@@ -835,11 +835,11 @@ felis_status felis_batch_create(const felis_params* const* instances, int32_t n,
       tabs.insert(tabs.end(), t.begin(), t.end());
     }
     if (e == cudaSuccess) e = cudaMalloc(&I.adi, tabs.size() * sizeof(float2));
-    if (e == cudaSuccess) e = cudaMemcpy(I.adi, tabs.data(), tabs.size() * sizeof(float2), cudaMemcpyHostToDevice);
+    if (e == cudaSuccess) e = to_device(I.adi, tabs.data(), tabs.size() * sizeof(float2), b->st);
     if (e == cudaSuccess) e = cudaMalloc(&I.part_e, (size_t)S * 2 * H * sizeof(double));
     if (e == cudaSuccess) e = cudaMalloc(&I.part_b, (size_t)S * (8 + 2 * H) * sizeof(double));
     if (e == cudaSuccess) e = cudaMalloc(&I.err, ERR_SLOTS * sizeof(int));
-    if (e == cudaSuccess) e = cudaMemset(I.err, 0, ERR_SLOTS * sizeof(int));
+    if (e == cudaSuccess) e = cudaMemsetAsync(I.err, 0, ERR_SLOTS * sizeof(int), b->st);
     if (e == cudaSuccess) e = cudaMalloc(&I.soff, (size_t)(S + 1) * sizeof(int64_t));
     if (e == cudaSuccess) e = cudaMalloc(&I.weight, (size_t)S * sizeof(float));
     if (e != cudaSuccess) return bad(FELIS_CUDA_ERROR, cudaGetErrorString(e));
@@ -936,9 +936,9 @@ felis_status felis_batch_upload_particles(felis_batch* b, int32_t inst, const do
   }
   if (n) BCK(cudaMemcpyAsync(I.th, theta, n * sizeof(double), cudaMemcpyDefault, b->st));
   BCK(cudaStreamSynchronize(b->st));
-  BCK(cudaMemcpy(I.soff, slice_offsets, (S + 1) * sizeof(int64_t), cudaMemcpyHostToDevice));
+  BCK(to_device(I.soff, slice_offsets, (S + 1) * sizeof(int64_t), b->st));
   std::vector<float> w(weights, weights + S);
-  BCK(cudaMemcpy(I.weight, w.data(), S * sizeof(float), cudaMemcpyHostToDevice));
+  BCK(to_device(I.weight, w.data(), S * sizeof(float), b->st));
   I.uploaded = true;
   return FELIS_OK;
 }
@@ -1067,8 +1067,8 @@ felis_status felis_batch_run(felis_batch* b, int32_t it0, int32_t it1) {
     BCK(cudaMalloc(&b->d_steps, (size_t)(b->steps_cap + 1) * n * sizeof(BStep)));
     BCK(cudaMalloc(&b->d_rad, (size_t)(b->steps_cap + 1) * n * b->LF_max * b->nr_max * 2 * sizeof(double)));
   }
-  BCK(cudaMemcpy(b->d_steps, tab.data(), tab.size() * sizeof(BStep), cudaMemcpyHostToDevice));
-  BCK(cudaMemcpy(b->d_rad, rad.data(), rad.size() * sizeof(double), cudaMemcpyHostToDevice));
+  BCK(to_device(b->d_steps, tab.data(), tab.size() * sizeof(BStep), b->st));
+  BCK(to_device(b->d_rad, rad.data(), rad.size() * sizeof(double), b->st));
   BCK(cudaStreamSynchronize(b->st));
   const bool deposit0 = b->src_valid_it != it0;
   cudaGraph_t graph = nullptr;

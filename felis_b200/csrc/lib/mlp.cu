@@ -318,11 +318,11 @@ felis_status felis_mlp_create(int32_t n_in, int32_t width, int32_t n_out, uint64
   cudaGetDevice(&m->device);
   cudaError_t e = cudaStreamCreateWithFlags(&m->st, cudaStreamNonBlocking);
   if (e == cudaSuccess) e = cudaMalloc(&m->d_err, sizeof(int));
-  if (e == cudaSuccess) e = cudaMemset(m->d_err, 0, sizeof(int));
+  if (e == cudaSuccess) e = cudaMemsetAsync(m->d_err, 0, sizeof(int), m->st);
   float** fb[] = {&m->p, &m->grad, &m->m, &m->v};
   for (auto f : fb) {
     if (e == cudaSuccess) e = cudaMalloc(f, m->n_param * sizeof(float));
-    if (e == cudaSuccess) e = cudaMemset(*f, 0, m->n_param * sizeof(float));
+    if (e == cudaSuccess) e = cudaMemsetAsync(*f, 0, m->n_param * sizeof(float), m->st);
   }
   for (int l = 0; l < kLayers && e == cudaSuccess; ++l) {
     e = cudaMalloc(&m->wb[l], (size_t)r[l] * c[l] * sizeof(bf16));
@@ -341,7 +341,7 @@ felis_status felis_mlp_create(int32_t n_in, int32_t width, int32_t n_out, uint64
     for (int i = 0; i < m->rows_real[l]; ++i)
       for (int j = 0; j < m->cols_real[l]; ++j) h[m->w_off[l] + (size_t)i * c[l] + j] = nd(rng);
   }
-  e = cudaMemcpy(m->p, h.data(), h.size() * sizeof(float), cudaMemcpyHostToDevice);
+  e = to_device(m->p, h.data(), h.size() * sizeof(float), m->st);
   if (e != cudaSuccess) return bad(FELIS_CUDA_ERROR, cudaGetErrorString(e));
   if (refresh_bf16(m) != FELIS_OK) return bad(FELIS_CUDA_ERROR, m->err.c_str());
   *out = m;
@@ -396,9 +396,9 @@ felis_status felis_mlp_set_params(felis_mlp* m, const float* in) {
     for (int i = 0; i < m->rows_real[l]; ++i) h[m->b_off[l] + i] = in[k++];
   }
   MCK(cudaStreamSynchronize(m->st));
-  MCK(cudaMemcpy(m->p, h.data(), h.size() * sizeof(float), cudaMemcpyHostToDevice));
-  MCK(cudaMemset(m->m, 0, m->n_param * sizeof(float)));
-  MCK(cudaMemset(m->v, 0, m->n_param * sizeof(float)));
+  MCK(to_device(m->p, h.data(), h.size() * sizeof(float), m->st));
+  MCK(cudaMemsetAsync(m->m, 0, m->n_param * sizeof(float), m->st));
+  MCK(cudaMemsetAsync(m->v, 0, m->n_param * sizeof(float), m->st));
   m->steps = 0;
   return refresh_bf16(m);
 }

@@ -6,6 +6,15 @@
 
 namespace felis {
 
+// A host table to the device ahead of work on `st`: copied on that stream, and
+// there when the call returns.  cudaMemcpy runs on the default stream, for which
+// the non-blocking streams of handles, ensembles and networks do not wait, and
+// from pageable memory it returns once the bytes are staged.
+inline cudaError_t to_device(void* dst, const void* src, size_t bytes, cudaStream_t st) {
+  const cudaError_t e = cudaMemcpyAsync(dst, src, bytes, cudaMemcpyHostToDevice, st);
+  return e == cudaSuccess ? cudaStreamSynchronize(st) : e;
+}
+
 struct CopyPart {
   const void* src;
   void* dst;
