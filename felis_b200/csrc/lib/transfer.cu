@@ -70,7 +70,13 @@ cudaError_t HostStage::reserve(int threads) {
   for (int t = 0; t < threads; ++t)
     for (int s = 0; s < kSlots; ++s)
       if (e == cudaSuccess && !ev_[t][s]) e = cudaEventCreateWithFlags(&ev_[t][s], cudaEventDisableTiming);
-  if (e == cudaSuccess) threads_ = threads;
+  if (e == cudaSuccess) {
+    threads_ = threads;
+  } else {
+    cudaGetLastError();  // the copies go without slots
+    if (pinned_) cudaFreeHost(pinned_);
+    pinned_ = nullptr;
+  }
   return e;
 }
 
@@ -88,7 +94,14 @@ cudaError_t HostStage::run(const CopyPart* parts, int nparts, Mode mode, int dev
   const OnDevice here(device);
   if (here.status != cudaSuccess) return here.status;
   moved_ += mode == kDownWiden ? 2 * total : total;
-  const bool plain = !pinned_ && moved_ < kLockAfter;
+  // one thread per 4 MB (written, where that is more), as far as the machine has cores
+  const int cores = std::max(1, (int)std::thread::hardware_concurrency());
+  auto threads_for = [&](size_t bytes) { return (int)std::min<size_t>(std::min(kThreads, cores), (bytes >> 22) + 1); };
+  int threads = threads_for(total);
+  // without slots while they would cost more than they give, and where the
+  // machine has no page-locked memory for them
+  const bool plain = (!pinned_ && moved_ < kLockAfter) || reserve(threads) != cudaSuccess;
+  if (plain) threads = threads_for(2 * total);
   if (plain && mode != kDownWiden) {
     for (int p = 0; p < nparts; ++p) {
       if (!parts[p].bytes) continue;
@@ -98,10 +111,6 @@ cudaError_t HostStage::run(const CopyPart* parts, int nparts, Mode mode, int dev
     }
     return cudaStreamSynchronize(st);
   }
-  // one thread per 4 MB (written, where that is more), as far as the machine has cores
-  const int cores = std::max(1, (int)std::thread::hardware_concurrency());
-  const size_t share = plain ? 2 * total : total;
-  const int threads = (int)std::min<size_t>(std::min(kThreads, cores), (share >> 22) + 1);
   std::atomic<size_t> next{0};
   std::atomic<int> status{cudaSuccess};
   auto fail = [&](cudaError_t x) {
@@ -167,13 +176,8 @@ cudaError_t HostStage::run(const CopyPart* parts, int nparts, Mode mode, int dev
     work(0);
     for (std::thread& t : pool) t.join();
   };
-  if (plain) {
-    spread(widen_plain);
-  } else {
-    const cudaError_t e = reserve(threads);
-    if (e != cudaSuccess) return e;
-    spread(staged);
-  }
+  if (plain) spread(widen_plain);
+  else spread(staged);
   if (status != cudaSuccess) cudaStreamSynchronize(st);  // nothing stays in flight through the slots
   return (cudaError_t)status.load();
 }

@@ -76,3 +76,25 @@ def test_small_copies_lock_no_pages(lib, stage, how):
     assert _copy(lib, one, how, 16 * per) == (0, 0, True)
     assert lib.host_live() == 2
     lib.stage_free(one)
+
+
+@pytest.mark.parametrize("how", [DOWN, WIDEN, UP])
+def test_copies_go_without_slots_where_there_are_none(lib, stage, how):
+    """A machine without page-locked memory left still copies, and takes slots
+    again when it can."""
+    words = 20 * MB
+    lib.fail_host_allocations(1)
+    try:
+        for _ in range(2):
+            assert _copy(lib, stage, how, words) == (0, 0, True)
+        assert lib.host_live() == 0
+    finally:
+        lib.fail_host_allocations(0)
+    assert _copy(lib, stage, how, words) == (0, 0, True)
+    assert lib.host_live() == 1
+    # more slots than it has: those it had are given up, the copies go on
+    lib.fail_host_allocations(1)
+    try:
+        assert _copy(lib, stage, how, 36 * MB) == (0, 0, True)
+    finally:
+        lib.fail_host_allocations(0)
