@@ -20,9 +20,9 @@
 
 #include <algorithm>
 #include <atomic>
+#include <exception>
 #include <memory>
 #include <new>
-#include <system_error>
 #include <thread>
 #include <vector>
 
@@ -167,14 +167,15 @@ cudaError_t HostStage::run(const CopyPart* parts, int nparts, Mode mode, int dev
       if (busy[k]) finish(k);
   };
   auto spread = [&](auto work) {
-    std::vector<std::thread> pool;
+    std::thread pool[kThreads];
+    int made = 0;
     try {
-      for (int t = 1; t < threads; ++t) pool.emplace_back(work, t);
-    } catch (const std::system_error&) {
+      for (; made < threads - 1; ++made) pool[made] = std::thread(work, made + 1);
+    } catch (const std::exception&) {
       // fewer threads: the chunks go to those that started
     }
     work(0);
-    for (std::thread& t : pool) t.join();
+    for (int t = 0; t < made; ++t) pool[t].join();
   };
   if (plain) spread(widen_plain);
   else spread(staged);
@@ -183,11 +184,19 @@ cudaError_t HostStage::run(const CopyPart* parts, int nparts, Mode mode, int dev
 }
 
 cudaError_t HostStage::download(const CopyPart* parts, int nparts, bool widen, int device, cudaStream_t st) {
-  return run(parts, nparts, widen ? kDownWiden : kDown, device, st);
+  try {
+    return run(parts, nparts, widen ? kDownWiden : kDown, device, st);
+  } catch (const std::bad_alloc&) {
+    return cudaErrorMemoryAllocation;
+  }
 }
 
 cudaError_t HostStage::upload(const CopyPart* parts, int nparts, int device, cudaStream_t st) {
-  return run(parts, nparts, kUp, device, st);
+  try {
+    return run(parts, nparts, kUp, device, st);
+  } catch (const std::bad_alloc&) {
+    return cudaErrorMemoryAllocation;
+  }
 }
 
 }  // namespace felis
