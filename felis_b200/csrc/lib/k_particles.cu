@@ -419,6 +419,11 @@ __device__ __forceinline__ void prep_one(const ParticleLaunch& a, int64_t n, dou
   D.rkey[n] = rk;
 }
 
+// e^{i phase} of a phase that nothing has wrapped: the reduction of fm::sincos
+// loses accuracy from 2^20 pi/2 on.  A call of its own, so that the usual phases
+// do not carry its code.
+__device__ __noinline__ void far_phase(double phase, double* s, double* c) { sincos(phase, s, c); }
+
 // Deterministic block sum of `v` (fixed shuffle tree, then warps in order).
 __device__ __forceinline__ double block_sum(double v, double* red) {
   for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
@@ -507,7 +512,10 @@ __global__ void __launch_bounds__(256, HM == 1 ? 4 : 3) k_particles(const __grid
         const int h = (q0 + k) >> 1;
         if (h >= G.H) break;
         const int H = G.harmony[h];
-        const cd e = H == 1 ? e1 : cexpi(-1.0 * H * th);
+        const double a = -1.0 * H * th;
+        cd e;
+        if (fabs(a) < 0x1p20) e = H == 1 ? e1 : cexpi(a);
+        else far_phase(a, &e.im, &e.re);
         part[k][t] = e.re * mw;
         part[k + 1][t] = -e.im * mw;
       }
