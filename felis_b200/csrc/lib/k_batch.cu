@@ -854,26 +854,30 @@ __global__ void __launch_bounds__(WIDE ? PushWide<HM>::value : kPushThreads, WID
   unsigned char* area = sm + o2;
   const size_t area_bytes = (size_t)a.smem_bytes - o2;
   // deposit statistics of the (pushed) beam: cell box and fixed-point bounds.
-  // The bounds are conservative and free of per-particle divisions: the 2-D
-  // term |w mc| / weight <= max(fb) / min|g| per thread (w <= 1); the radial term
+  // The 2-D term |w mc| / weight <= fb / |g| (w <= 1).  With odd harmonics alone fb
+  // is 1 and the least |g| gives the bound; an even one takes a quotient per
+  // particle, beside its square root and arc tangent.  (The largest fb over the
+  // least |g|, of other particles, made the quantum up to their spread coarser.)
+  // The largest value over the slice does not depend on which thread has which
+  // particle.  The radial term
   // (1 + |wr1|) / max(ir, 1) <= 1.625 (|wr1| <= 5/8 for ir >= 1), counted when
   // a particle may lie inside the radial grid.
   int ci0 = 1 << 30, ci1 = -(1 << 30), cj0 = 1 << 30, cj1 = -(1 << 30);
-  float wfmax = 0.f, gmin = 3.0e38f;
+  float wfmax = 0.f, gmin = 3.0e38f;  // largest fb / |g| of even harmonics, least |g|
   int rin = 0;
   const float rlim2 = ((float)nr + 0.5f) * dr * ((float)nr + 0.5f) * dr;
   auto stats = [&](auto even_c, int ii, int jj, float x, float y, float px, float py, float g) {
     if (ii >= 0 && ii < nx && jj >= 0 && jj < ny) {
       ci0 = min(ci0, ii); ci1 = max(ci1, ii); cj0 = min(cj0, jj); cj1 = max(cj1, jj);
-      float fb = 1.f;  // odd harmonics accumulate w mc (|f| applied later); bilinear w <= 1
+      // odd harmonics accumulate w mc (|f| applied later): fb = 1
       if constexpr (decltype(even_c)::value) {
         float xi2;
         float2 eP;
         pol_phase(D.K0, D.ue, D.K0a, D.Phi_half, px, py, &xi2, &eP);
-        fb = fmaxf(fb, 2.f * xi2 * Hmax);
+        wfmax = fmaxf(wfmax, fmaxf(1.f, 2.f * xi2 * Hmax) / fabsf(g));
+      } else {
+        gmin = fminf(gmin, fabsf(g));
       }
-      wfmax = fmaxf(wfmax, fb);
-      gmin = fminf(gmin, fabsf(g));
     }
     rin |= (x * x + y * y < rlim2) ? 1 : 0;
   };
@@ -1268,7 +1272,7 @@ __global__ void __launch_bounds__(WIDE ? PushWide<HM>::value : kPushThreads, WID
       for (int k = 0; k < 3; ++k) u[k] = fmaxf(u[k], rbnd2[q][k]);
     }
     mi0 = t[0]; mi1 = -t[1]; mj0 = t[2]; mj1 = -t[3];
-    bmx = u[0] > 0.f ? u[0] / -u[2] : 0.f;
+    bmx = fmaxf(u[0], -u[2] < 3.0e38f ? 1.f / -u[2] : 0.f);
     rmx = u[1];
   }
   const float tb = bmx * 1.0625f * Hmax * weight * fabsf(D.coef_U), bnd = tb * (float)P;
