@@ -301,35 +301,27 @@ bool prep_coef(const felis_handle* h, const felis_lattice& L, PrepCoef* c) {
 // ADI coefficient tables of one harmonic (solveField.cpp:112-181).
 void build_adi(felis_handle* h, int hidx, const std::vector<cd>& al, const std::vector<cd>& alP,
                const std::vector<cd>& be, const std::vector<cd>& beP, std::vector<cd>& cv, std::vector<double>& dv,
-               size_t offs_c[14], size_t offs_d[6]) {
+               size_t offs_c[10], size_t offs_d[6]) {
   const int nx = h->p.nx, ny = h->p.ny;
   const double H = (double)h->p.harmony[hidx];
-  // layout: complex arrays rx_m, rx_0, rx_p (ny), ax_p, ax_a, ax_q, ax_cc (nx),
-  //         ry_m, ry_0, ry_p (nx), ay_p, ay_a, ay_q, ay_cc (ny)
-  const int sizes_c[14] = {ny, ny, ny, nx, nx, nx, nx, nx, nx, nx, ny, ny, ny, ny};
+  // layout: complex arrays rx_0 (ny), ax_p, ax_a, ax_q, ax_cc (nx),
+  //         ry_0 (nx), ay_p, ay_a, ay_q, ay_cc (ny)
+  const int sizes_c[10] = {ny, nx, nx, nx, nx, nx, ny, ny, ny, ny};
   size_t o = 0;
-  for (int k = 0; k < 14; ++k) { offs_c[k] = o; o += sizes_c[k]; }
+  for (int k = 0; k < 10; ++k) { offs_c[k] = o; o += sizes_c[k]; }
   cv.assign(o, C(0, 0));
   const int sizes_d[6] = {nx, nx, nx, ny, ny, ny};  // ax_pinv, ax_qinv, ax_ccinv, ay_*
   o = 0;
   for (int k = 0; k < 6; ++k) { offs_d[k] = o; o += sizes_d[k]; }
   dv.assign(o, 0.0);
-  cd* rx_m = &cv[offs_c[0]]; cd* rx_0 = &cv[offs_c[1]]; cd* rx_p = &cv[offs_c[2]];
-  cd* ax_p = &cv[offs_c[3]]; cd* ax_a = &cv[offs_c[4]]; cd* ax_q = &cv[offs_c[5]]; cd* ax_cc = &cv[offs_c[6]];
-  cd* ry_m = &cv[offs_c[7]]; cd* ry_0 = &cv[offs_c[8]]; cd* ry_p = &cv[offs_c[9]];
-  cd* ay_p = &cv[offs_c[10]]; cd* ay_a = &cv[offs_c[11]]; cd* ay_q = &cv[offs_c[12]]; cd* ay_cc = &cv[offs_c[13]];
+  cd* rx_0 = &cv[offs_c[0]];
+  cd* ax_p = &cv[offs_c[1]]; cd* ax_a = &cv[offs_c[2]]; cd* ax_q = &cv[offs_c[3]]; cd* ax_cc = &cv[offs_c[4]];
+  cd* ry_0 = &cv[offs_c[5]];
+  cd* ay_p = &cv[offs_c[6]]; cd* ay_a = &cv[offs_c[7]]; cd* ay_q = &cv[offs_c[8]]; cd* ay_cc = &cv[offs_c[9]];
   double* ax_pinv = &dv[offs_d[0]]; double* ax_qinv = &dv[offs_d[1]]; double* ax_ccinv = &dv[offs_d[2]];
   double* ay_pinv = &dv[offs_d[3]]; double* ay_qinv = &dv[offs_d[4]]; double* ay_ccinv = &dv[offs_d[5]];
-  for (int j = 1; j < ny - 1; ++j) {
-    rx_m[j] = cneg(beP[j]);
-    rx_0[j] = cadd(cradd(H, beP[j]), be[j]);
-    rx_p[j] = be[j];
-  }
-  for (int i = 1; i < nx - 1; ++i) {
-    ry_m[i] = cneg(alP[i]);
-    ry_0[i] = cadd(cradd(H, alP[i]), al[i]);
-    ry_p[i] = al[i];
-  }
+  for (int j = 1; j < ny - 1; ++j) rx_0[j] = cadd(cradd(H, beP[j]), be[j]);
+  for (int i = 1; i < nx - 1; ++i) ry_0[i] = cadd(cradd(H, alP[i]), al[i]);
   // x recurrence
   std::vector<cd> CC(nx, C(0, 0));
   CC[1] = cdiv(csub(crsub(H, alP[1]), al[1]), alP[1]);
@@ -480,9 +472,6 @@ felis_status run_deposit(felis_handle* h, const felis_lattice& L) {
   d.chunk2 = h->dep_plan.chunk2;
   d.chunkr = h->dep_plan.chunkr;
   d.radial = h->d_radial;
-  d.neven = 0;
-  for (int k = 0; k < h->p.num_harmony; ++k) d.neven += (h->p.harmony[k] % 2 == 0);
-  d.err = h->d_err;
   {
     KernelScope ks(h, FELIS_KERNEL_DEPOSIT);
     if (!(h->radial_A == d.A)) {
@@ -760,7 +749,7 @@ felis_status felis_create(const felis_params* p, felis_handle** out) {
     for (int k = 0; k < H && st == FELIS_OK; ++k) {
       std::vector<cd> cv;
       std::vector<double> dv;
-      size_t oc[14], od[6];
+      size_t oc[10], od[6];
       build_adi(h, k, al, alP, be, beP, cv, dv, oc, od);
       cd* dc = nullptr;
       double* dd = nullptr;
@@ -773,10 +762,10 @@ felis_status felis_create(const felis_params* p, felis_handle** out) {
       h->adi_dev.push_back(dc);
       h->adi_dev.push_back(dd);
       AdiTab& T = tabs[k];
-      T.rx_m = dc + oc[0]; T.rx_0 = dc + oc[1]; T.rx_p = dc + oc[2];
-      T.ax_p = dc + oc[3]; T.ax_a = dc + oc[4]; T.ax_q = dc + oc[5]; T.ax_cc = dc + oc[6];
-      T.ry_m = dc + oc[7]; T.ry_0 = dc + oc[8]; T.ry_p = dc + oc[9];
-      T.ay_p = dc + oc[10]; T.ay_a = dc + oc[11]; T.ay_q = dc + oc[12]; T.ay_cc = dc + oc[13];
+      T.rx_0 = dc + oc[0];
+      T.ax_p = dc + oc[1]; T.ax_a = dc + oc[2]; T.ax_q = dc + oc[3]; T.ax_cc = dc + oc[4];
+      T.ry_0 = dc + oc[5];
+      T.ay_p = dc + oc[6]; T.ay_a = dc + oc[7]; T.ay_q = dc + oc[8]; T.ay_cc = dc + oc[9];
       T.ax_pinv = dd + od[0]; T.ax_qinv = dd + od[1]; T.ax_ccinv = dd + od[2];
       T.ay_pinv = dd + od[3]; T.ay_qinv = dd + od[4]; T.ay_ccinv = dd + od[5];
     }

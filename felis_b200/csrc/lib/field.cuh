@@ -9,14 +9,14 @@ namespace felis {
 // 110-181), built on the host with the same complex formulas as the CPU
 // restatement so the recurrences below reproduce it bit for bit.
 struct AdiTab {
-  // x-sweep right-hand side (index j): -betaP, (H + betaP + beta), beta
-  const cd *rx_m, *rx_0, *rx_p;
+  // x-sweep right-hand side (index j): H + betaP + beta (betaP and beta below)
+  const cd* rx_0;
   // x-sweep recurrence (index i): alphaP and 1/|alphaP|^2, alpha,
   // Q = alphaP*CC[i-1] and 1/|Q|^2, CC and 1/|CC|^2
   const cd *ax_p, *ax_a, *ax_q, *ax_cc;
   const double *ax_pinv, *ax_qinv, *ax_ccinv;
-  // y-sweep right-hand side (index i): -alphaP, (H + alphaP + alpha), alpha
-  const cd *ry_m, *ry_0, *ry_p;
+  // y-sweep right-hand side (index i): H + alphaP + alpha
+  const cd* ry_0;
   // y-sweep recurrence (index j)
   const cd *ay_p, *ay_a, *ay_q, *ay_cc;
   const double *ay_pinv, *ay_qinv, *ay_ccinv;
@@ -50,10 +50,8 @@ struct DepositLaunch {
   double2 fconst[FELIS_MAX_HARMONY][2];  // odd-harmonic fx, fy (per call constants)
   cd etaX, etaY;
   double A;             // Ez Thomas coefficient (solveField.cpp:320)
-  int neven;            // number of even harmonics
   int chunk2, chunkr;   // particles per chunk of the 2-D and the radial sums (DepositPlan)
   const double2* radial;  // [L*F][nr] radial elimination for A (launch_radial_elimination)
-  int* err;
 };
 
 // Chunk sizes and shared memory of the deposit; false when the radial grid is
