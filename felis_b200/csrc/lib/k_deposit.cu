@@ -15,10 +15,13 @@
 // lanes of its pairs.  A popcount below the lane's own bit is the particle's
 // rank in the group, and a counter per target and warp carries the rank on
 // from group to group.  A prefix sum over targets and warps turns the ranks
-// into places.  No sort and no merge, whatever the number of cells.
+// into places.  No sort and no merge.
 //
 // The block's targets are cut into bands of rows (2-D) or of bins (r) that
 // fit the counters; the band of a usual beam (33 x 33 cells) is the whole box.
+// Every band walks the slice's particles: a 1 GeV beam on 152 x 152 points (a box
+// of about 145 x 145, 13 bands) takes 0.64 ms for a slice of 8192 particles and
+// 0.79 for 64 of them (1.14 and 1.26 with the sort).
 //
 // Measured (B200, 8192 particles per slice, 102 x 102): a single slice 0.415 ms
 // with a stable radix sort per chunk and a four-way merge per cell, 0.076 ms

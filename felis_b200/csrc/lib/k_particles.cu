@@ -2,8 +2,9 @@
 //
 // Compiled with --fmad=false: every expression below is evaluated with the
 // operand order of the reference (particlePush.cpp, solveField.cpp,
-// rearrangeParticles.cpp) and no contraction, so the results equal the CPU
-// restatement bit for bit.  One thread owns one particle; a block owns one
+// rearrangeParticles.cpp) and no contraction, so particles and fields equal the
+// CPU restatement bit for bit (the diagnostics' sums have an order and sines of
+// their own: last bits).  One thread owns one particle; a block owns one
 // tile of <= 256 consecutive particles of one (species, slice), so the
 // slice's field plane, weight and wake term are uniform per block.
 //
