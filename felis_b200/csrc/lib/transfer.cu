@@ -98,9 +98,11 @@ cudaError_t HostStage::run(const CopyPart* parts, int nparts, Mode mode, int dev
   const int cores = std::max(1, (int)std::thread::hardware_concurrency());
   auto threads_for = [&](size_t bytes) { return (int)std::min<size_t>(std::min(kThreads, cores), (bytes >> 22) + 1); };
   int threads = threads_for(total);
-  // without slots while they would cost more than they give, and where the
-  // machine has no page-locked memory for them
-  const bool plain = (!pinned_ && moved_ < kLockAfter) || reserve(threads) != cudaSuccess;
+  // without slots while they would cost more than they give (a call of less than
+  // one chunk makes none, however often it comes), and where the machine has no
+  // page-locked memory for them
+  const bool small = total < kChunk && mode != kDownWiden;
+  const bool plain = (!pinned_ && (small || moved_ < kLockAfter)) || reserve(threads) != cudaSuccess;
   if (plain) threads = threads_for(2 * total);
   if (plain && mode != kDownWiden) {
     for (int p = 0; p < nparts; ++p) {

@@ -98,3 +98,13 @@ def test_copies_go_without_slots_where_there_are_none(lib, stage, how):
         assert _copy(lib, stage, how, 36 * MB) == (0, 0, True)
     finally:
         lib.fail_host_allocations(0)
+
+
+@pytest.mark.parametrize("how", [DOWN, UP])
+def test_small_calls_never_lock_pages(lib, stage, how):
+    """A call of less than a chunk gains nothing from slots, after any number of them."""
+    for _ in range(90):
+        assert _copy(lib, stage, how, MB // 4 - 5) == (0, 0, True)
+    assert lib.host_live() == 0
+    assert _copy(lib, stage, how, MB) == (0, 0, True)
+    assert lib.host_live() == 1
